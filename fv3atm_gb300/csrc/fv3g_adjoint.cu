@@ -152,21 +152,183 @@ __device__ T ppm_face(int hord, double lim_fac, int f, const XF& X, const DF& DX
   return high ? (X(f) + T(w1) * bl[1]) - T(w2) * (bl[1] + br[1]) : X(f);
 }
 
-// The six weights of face f's flux on cells f-3..f+2 (one forward-mode pass
-// per cell) and the flux value.
-template <class XV, class DF>
-__device__ __forceinline__ double face_weights(int hord, double lim_fac, int f, const XV& xv, const DF& DX, double c,
-                                               int eLo, int eHi, double* w, long long ws) {
-  double val = 0.0;
-#pragma unroll 1
-  for (int s = 0; s < 6; ++s) {
-    const int ms = f - 3 + s;
-    auto X = [&](int m) -> D2 { return D2(xv(m), m == ms ? 1.0 : 0.0); };
-    const D2 r = ppm_face<D2>(hord, lim_fac, f, X, DX, c, eLo, eHi);
-    w[s * ws] = r.d;
-    val = r.v;
+// Faces whose cells f-1 or f take a one-sided value at a cube-face edge e
+// (cells e-2 .. e+1 do), in the sweeps' lines.
+__device__ __forceinline__ bool edge_face(int f, int eLo, int eHi) {
+  return (eLo != NO_EDGE && f >= eLo - 2 && f <= eLo + 2) || (eHi != NO_EDGE && f >= eHi - 2 && f <= eHi + 2);
+}
+
+// The six weights of face f's flux on cells f-3..f+2 and the flux value, away
+// from cube-face edges, in closed form: the flux reads the upwind cell m, its
+// deviations bl, br and (hord 1, 5) the filter tests of both cells, and every
+// branch leaves a linear form of the means, so one evaluation of the values
+// and about twenty multiply-adds replace a forward-mode pass per cell.  FP64
+// runs at 1/64 of the FP32 rate, so the count of FP64 operations is the cost:
+// six C96 tiles x 64 levels x 4 tracers, hord 5, six substeps took 505 ms in
+// both kernels with six passes per face.  The branch conventions are those of
+// ppm_face on dual numbers (on a tie the later operand).
+__device__ __forceinline__ void put_weights(double* w, long long ws, const double* W) {
+#pragma unroll
+  for (int s = 0; s < 6; ++s) w[s * ws] = W[s];
+}
+
+// Slope of the middle cell of (xm, x0, xp) and its derivatives p on the three.
+__device__ __forceinline__ double slope_grad(double xm, double x0, double xp, double* p) {
+  const double xt = 0.25 * (xp - xm), ax = fabs(xt);
+  const double hi1 = xm > x0 ? xm : x0, lo1 = xm < x0 ? xm : x0;
+  const bool hi_m = xm > x0 && hi1 > xp, hi_0 = !(xm > x0) && hi1 > xp;  // else xp is the largest
+  const bool lo_m = xm < x0 && lo1 < xp, lo_0 = !(xm < x0) && lo1 < xp;
+  const double up = (hi1 > xp ? hi1 : xp) - x0, dn = x0 - (lo1 < xp ? lo1 : xp);
+  const double m1 = ax < up ? ax : up;
+  const bool use_dn = !(m1 < dn), use_up = !use_dn && !(ax < up);
+  const double mag = use_dn ? dn : m1;
+  const bool neg = signbit(mag) != signbit(xt);
+  const double sg = neg ? -1.0 : 1.0;
+  if (use_dn) {
+    p[0] = lo_m ? -sg : 0.0;
+    p[1] = lo_0 ? 0.0 : sg;
+    p[2] = (lo_m || lo_0) ? 0.0 : -sg;
+  } else if (use_up) {
+    p[0] = hi_m ? sg : 0.0;
+    p[1] = hi_0 ? 0.0 : -sg;
+    p[2] = (hi_m || hi_0) ? 0.0 : sg;
+  } else {
+    p[0] = -0.25;
+    p[1] = 0.0;
+    p[2] = 0.25;
+    return xt;  // |xt| with the sign of xt
   }
-  return val;
+  return neg ? -mag : mag;
+}
+
+template <class XV>
+__device__ __forceinline__ double face_weights(int hord, double lim_fac, int f, const XV& xv, double c, double* w,
+                                               long long ws) {
+  double x[6], W[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int s = 0; s < 6; ++s) x[s] = xv(f - 3 + s);
+  const bool left = c > 0.0;  // upwind cell f-1 (window cell 2), else f (window cell 3)
+  const double ac = fabs(c), w1 = 1.0 - ac, w2 = ac * w1;
+  const double cl = left ? -w2 : w1 - w2, cr = left ? w1 - w2 : -w2;  // flux = x_m + cl bl + cr br
+  if (hord == 8) {
+    double y[5], p0[3], p1[3], p2[3], V[5];  // cells m-2 .. m+2
+#pragma unroll
+    for (int s = 0; s < 5; ++s) y[s] = left ? x[s] : x[s + 1];
+    const double d0 = slope_grad(y[0], y[1], y[2], p0), d1 = slope_grad(y[1], y[2], y[3], p1),
+                 d2 = slope_grad(y[2], y[3], y[4], p2);
+    const double xt = d1 + d1, axt = fabs(xt);
+    const double tl = (0.5 * (y[1] + y[2]) + (d0 - d1) * (1.0 / 3.0)) - y[2];
+    const double tr = (0.5 * (y[2] + y[3]) + (d1 - d2) * (1.0 / 3.0)) - y[2];
+    const bool lim_l = axt < fabs(tl), lim_r = axt < fabs(tr);
+    const double bl = copysign(lim_l ? axt : fabs(tl), -xt), br = copysign(lim_r ? axt : fabs(tr), xt);
+    // derivatives of bl: -2 dm where limited, else those of +-tl; br likewise
+    const double kl = cl * ((signbit(tl) != signbit(-xt)) ? -1.0 : 1.0);
+    const double kr = cr * ((signbit(tr) != signbit(xt)) ? -1.0 : 1.0);
+    const double hl = lim_l ? 0.0 : 0.5 * kl, hr = lim_r ? 0.0 : 0.5 * kr;
+    const double gl = lim_l ? 0.0 : kl * (1.0 / 3.0), gr = lim_r ? 0.0 : kr * (1.0 / 3.0);
+    const double g1 = (lim_l ? -2.0 * cl : -gl) + (lim_r ? 2.0 * cr : gr);
+    V[0] = gl * p0[0];
+    V[1] = hl + gl * p0[1] + g1 * p1[0];
+    V[2] = (1.0 - hl - hr) + gl * p0[2] + g1 * p1[1] - gr * p2[0];
+    V[3] = hr + g1 * p1[2] - gr * p2[1];
+    V[4] = -gr * p2[2];
+#pragma unroll
+    for (int s = 0; s < 6; ++s) W[s] = left ? (s < 5 ? V[s] : 0.0) : (s > 0 ? V[s - 1] : 0.0);
+    put_weights(w, ws, W);
+    return (y[2] + w1 * (left ? br : bl)) - w2 * (bl + br);
+  }
+  double al[3], bl[2], br[2];
+#pragma unroll
+  for (int g = 0; g < 3; ++g) al[g] = (7.0 / 12.0) * (x[g + 1] + x[g + 2]) - (1.0 / 12.0) * (x[g] + x[g + 3]);
+  bool high = false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    bl[h] = al[h] - x[h + 2];
+    br[h] = al[h + 1] - x[h + 2];
+    high = high || (hord == 5 ? bl[h] * br[h] < 0.0 : fabs(lim_fac * (bl[h] + br[h])) < fabs(bl[h] - br[h]));
+  }
+  const double xu = left ? x[2] : x[3];
+  const double a = high ? cl : 0.0, b = high ? cr : 0.0;
+  const double va = (-1.0 / 12.0) * a, vb = (-1.0 / 12.0) * b, ua = (7.0 / 12.0) * a, ub = (7.0 / 12.0) * b;
+  const double V[5] = {va, ua + vb, 1.0 + (ua + ub - a - b), va + ub, vb};
+#pragma unroll
+  for (int s = 0; s < 6; ++s) W[s] = left ? (s < 5 ? V[s] : 0.0) : (s > 0 ? V[s - 1] : 0.0);
+  put_weights(w, ws, W);
+  const double bu = left ? bl[0] : bl[1], ru = left ? br[0] : br[1];
+  return high ? (xu + w1 * (left ? ru : bu)) - w2 * (bu + ru) : xu;
+}
+
+// The same beside a cube-face edge.  hord 1 / 5: the interfaces' taps, the
+// one-sided ones included.  hord 8: one forward-mode pass of ppm_face per
+// cell (six faces of a line).
+template <class XV, class DF>
+__device__ double edge_face_weights(int hord, double lim_fac, int f, const XV& xv, const DF& DX, double c, int eLo,
+                                    int eHi, double* w, long long ws) {
+  if (hord == 8) {
+    double val = 0.0;
+#pragma unroll 1
+    for (int s = 0; s < 6; ++s) {
+      const int ms = f - 3 + s;
+      auto X = [&](int m) -> D2 { return D2(xv(m), m == ms ? 1.0 : 0.0); };
+      const D2 r = ppm_face<D2>(hord, lim_fac, f, X, DX, c, eLo, eHi);
+      w[s * ws] = r.d;
+      val = r.v;
+    }
+    return val;
+  }
+  double x[6];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) x[s] = xv(f - 3 + s);
+  double G[3][6], al[3];  // taps on the window and values of interfaces f-1, f, f+1
+#pragma unroll
+  for (int g = 0; g < 3; ++g) {
+    const int u = f - 1 + g;
+    double t[4] = {-1.0 / 12.0, 7.0 / 12.0, 7.0 / 12.0, -1.0 / 12.0};
+    int base = u - 2;
+    for (int side = 0; side < 2; ++side) {  // the high edge's one-sided values take precedence
+      const int e = side ? eHi : eLo;
+      if (e == NO_EDGE) continue;
+      if (u == e - 1) {
+        base = e - 3;
+        t[0] = kC1; t[1] = kC2; t[2] = kC3; t[3] = 0.0;
+      } else if (u == e) {
+        base = e - 2;
+        const double d2 = DX(e - 2), d1 = DX(e - 1), d0 = DX(e), d3 = DX(e + 1);
+        t[0] = -0.5 * d1 / (d2 + d1);
+        t[1] = 0.5 * (2.0 * d1 + d2) / (d2 + d1);
+        t[2] = 0.5 * (2.0 * d0 + d3) / (d0 + d3);
+        t[3] = -0.5 * d0 / (d0 + d3);
+      } else if (u == e + 1) {
+        base = e;
+        t[0] = kC3; t[1] = kC2; t[2] = kC1; t[3] = 0.0;
+      }
+    }
+    al[g] = 0.0;
+#pragma unroll
+    for (int s = 0; s < 6; ++s) {
+      const int k = f - 3 + s - base;
+      G[g][s] = k == 0 ? t[0] : k == 1 ? t[1] : k == 2 ? t[2] : k == 3 ? t[3] : 0.0;
+      al[g] += G[g][s] * x[s];
+    }
+  }
+  bool high = false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const double bl = al[h] - x[h + 2], br = al[h + 1] - x[h + 2];
+    high = high || (hord == 5 ? bl * br < 0.0 : fabs(lim_fac * (bl + br)) < fabs(bl - br));
+  }
+  const bool left = c > 0.0;
+  const double ac = fabs(c), w1 = 1.0 - ac, w2 = ac * w1;
+  const double a = high ? (left ? -w2 : w1 - w2) : 0.0, b = high ? (left ? w1 - w2 : -w2) : 0.0;
+  const double xu = left ? x[2] : x[3];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) {
+    const double Ga = left ? G[0][s] : G[1][s], Gb = left ? G[1][s] : G[2][s];
+    const bool up = s == (left ? 2 : 3);
+    w[s * ws] = a * Ga + b * Gb + (up ? (1.0 - a) - b : 0.0);
+  }
+  const double bl = (left ? al[0] : al[1]) - xu, br = (left ? al[1] : al[2]) - xu;
+  return high ? (xu + w1 * (left ? br : bl)) - w2 * (bl + br) : xu;
 }
 
 // ------------------------------------------------------- plane indexing ---
@@ -251,32 +413,64 @@ __global__ void k_lin_corners(const LinArgs a, const double* q, double* c1, doub
 
 // Inner sweeps: y faces for every column of the data domain on the dir-2
 // copy, x faces for every row on the dir-1 copy: weights and flux values.
+// Faces beside a cube-face edge are left to k_lin_edges.
 __global__ void k_lin_inner(const LinArgs a, const LinTraj tr) {
   Cell c;
   if (!cell_of(a, c)) return;
   const long long ws = (long long)a.nt * a.nq * a.npz * a.P;
   const PlaneGeom& pg = a.pg;
-  double fy = 0.0, fx = 0.0;
-  if (yi_face(a, c.i, c.j)) {
-    const double* line = tr.qc2 + c.q0;
-    const int i = c.i;
-    auto xv = [&](int m) { return line[pg.at(i, m)]; };
-    auto dx = [&](int m) { return a.dya[c.met + pg.at(i, m)]; };
-    fy = face_weights(a.hord, a.lim_fac, c.j, xv, dx, a.cy[c.lev + c.p], a.es, a.en, tr.wyi + c.q0 + c.p, ws);
-  } else {
+  if (!yi_face(a, c.i, c.j)) {
     for (int s = 0; s < 6; ++s) tr.wyi[s * ws + c.q0 + c.p] = 0.0;
+    tr.fy2[c.q0 + c.p] = 0.0;
+  } else if (!edge_face(c.j, a.es, a.en)) {
+    const double* line = tr.qc2 + c.q0;
+    auto xv = [&](int m) { return line[pg.at(c.i, m)]; };
+    tr.fy2[c.q0 + c.p] =
+        face_weights(a.hord, a.lim_fac, c.j, xv, a.cy[c.lev + c.p], tr.wyi + c.q0 + c.p, ws);
   }
-  if (xi_face(a, c.i, c.j)) {
-    const double* line = tr.qc1 + c.q0;
-    const int j = c.j;
-    auto xv = [&](int m) { return line[pg.at(m, j)]; };
-    auto dx = [&](int m) { return a.dxa[c.met + pg.at(m, j)]; };
-    fx = face_weights(a.hord, a.lim_fac, c.i, xv, dx, a.cx[c.lev + c.p], a.ew, a.ee, tr.wxi + c.q0 + c.p, ws);
-  } else {
+  if (!xi_face(a, c.i, c.j)) {
     for (int s = 0; s < 6; ++s) tr.wxi[s * ws + c.q0 + c.p] = 0.0;
+    tr.fx2[c.q0 + c.p] = 0.0;
+  } else if (!edge_face(c.i, a.ew, a.ee)) {
+    const double* line = tr.qc1 + c.q0;
+    auto xv = [&](int m) { return line[pg.at(m, c.j)]; };
+    tr.fx2[c.q0 + c.p] =
+        face_weights(a.hord, a.lim_fac, c.i, xv, a.cx[c.lev + c.p], tr.wxi + c.q0 + c.p, ws);
   }
-  tr.fy2[c.q0 + c.p] = fy;
-  tr.fx2[c.q0 + c.p] = fx;
+}
+
+// Faces beside the cube-face edges of both sweeps of a pass (inner: x on the
+// dir-1 copy, y on the dir-2 copy; outer: x on q_i, y on q_j), a thread per
+// line, edge and face around it (10 faces of a line): compact, so that the
+// few one-sided faces do not hold up warps of ordinary ones.  blockIdx.z: 0 x
+// faces, 1 y faces.
+__global__ void k_lin_edges(const LinArgs a, const LinTraj tr, int outer) {
+  const bool ydir = blockIdx.z == 1;
+  const int lo = ydir ? (outer ? a.is : a.isd) : (outer ? a.js : a.jsd);
+  const int hi = ydir ? (outer ? a.ie : a.ied) : (outer ? a.je : a.jed);
+  const int nlines = hi - lo + 1;
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= nlines * 10) return;
+  const int line = lo + id % nlines, slot = id / nlines;
+  const int eLo = ydir ? a.es : a.ew, eHi = ydir ? a.en : a.ee;
+  const int e = slot < 5 ? eLo : eHi;
+  if (e == NO_EDGE) return;
+  const int f = e - 2 + slot % 5;
+  if (!in_rng(f, ydir ? a.js : a.is, (ydir ? a.je : a.ie) + 1)) return;
+  const PlaneGeom& pg = a.pg;
+  const long long ws = (long long)a.nt * a.nq * a.npz * a.P;
+  const int pl = blockIdx.y, per_tile = a.nq * a.npz;
+  const int t = pl / per_tile;
+  const long long q0 = (long long)pl * a.P, lev = ((long long)t * a.npz + pl % a.npz) * a.P, met = (long long)t * a.P;
+  const long long p = ydir ? pg.at(line, f) : pg.at(f, line);
+  const double* src = (outer ? (ydir ? tr.qj : tr.qi) : (ydir ? tr.qc2 : tr.qc1)) + q0;
+  const double* da = (ydir ? a.dya : a.dxa) + met;
+  double* w = (outer ? (ydir ? tr.wyo : tr.wxo) : (ydir ? tr.wyi : tr.wxi)) + q0 + p;
+  auto at = [&](int m) { return ydir ? pg.at(line, m) : pg.at(m, line); };
+  auto xv = [&](int m) { return src[at(m)]; };
+  auto dx = [&](int m) { return da[at(m)]; };
+  const double fl = edge_face_weights(a.hord, a.lim_fac, f, xv, dx, (ydir ? a.cy : a.cx)[lev + p], eLo, eHi, w, ws);
+  if (!outer) (ydir ? tr.fy2 : tr.fx2)[q0 + p] = fl;
 }
 
 // Inner updates: q_i = (q area + yfx fy2 - yfx' fy2') / ra_y on the compute
@@ -304,29 +498,25 @@ __global__ void k_lin_mid(const LinArgs a, const double* c1, const double* c2, c
 }
 
 // Outer sweeps: x faces of the compute rows on q_i, y faces of the compute
-// columns on q_j: weights.
+// columns on q_j: weights (faces beside a cube-face edge: k_lin_edges).
 __global__ void k_lin_outer(const LinArgs a, const LinTraj tr) {
   Cell c;
   if (!cell_of(a, c)) return;
   const long long ws = (long long)a.nt * a.nq * a.npz * a.P;
   const PlaneGeom& pg = a.pg;
-  if (xo_face(a, c.i, c.j)) {
-    const double* line = tr.qi + c.q0;
-    const int j = c.j;
-    auto xv = [&](int m) { return line[pg.at(m, j)]; };
-    auto dx = [&](int m) { return a.dxa[c.met + pg.at(m, j)]; };
-    face_weights(a.hord, a.lim_fac, c.i, xv, dx, a.cx[c.lev + c.p], a.ew, a.ee, tr.wxo + c.q0 + c.p, ws);
-  } else {
+  if (!xo_face(a, c.i, c.j)) {
     for (int s = 0; s < 6; ++s) tr.wxo[s * ws + c.q0 + c.p] = 0.0;
+  } else if (!edge_face(c.i, a.ew, a.ee)) {
+    const double* line = tr.qi + c.q0;
+    auto xv = [&](int m) { return line[pg.at(m, c.j)]; };
+    face_weights(a.hord, a.lim_fac, c.i, xv, a.cx[c.lev + c.p], tr.wxo + c.q0 + c.p, ws);
   }
-  if (yo_face(a, c.i, c.j)) {
-    const double* line = tr.qj + c.q0;
-    const int i = c.i;
-    auto xv = [&](int m) { return line[pg.at(i, m)]; };
-    auto dx = [&](int m) { return a.dya[c.met + pg.at(i, m)]; };
-    face_weights(a.hord, a.lim_fac, c.j, xv, dx, a.cy[c.lev + c.p], a.es, a.en, tr.wyo + c.q0 + c.p, ws);
-  } else {
+  if (!yo_face(a, c.i, c.j)) {
     for (int s = 0; s < 6; ++s) tr.wyo[s * ws + c.q0 + c.p] = 0.0;
+  } else if (!edge_face(c.j, a.es, a.en)) {
+    const double* line = tr.qj + c.q0;
+    auto xv = [&](int m) { return line[pg.at(c.i, m)]; };
+    face_weights(a.hord, a.lim_fac, c.j, xv, a.cy[c.lev + c.p], tr.wyo + c.q0 + c.p, ws);
   }
 }
 
@@ -795,9 +985,14 @@ int lin_unpack_tangent(const Dual<double>* in, double* d, long long n, cudaStrea
 int lin_trajectory(const LinArgs& a, const double* q, const LinTraj& tr, cudaStream_t s) {
   const dim3 g = plane_grid(a);
   k_lin_corners<<<g, 128, 0, s>>>(a, q, tr.qc1, tr.qc2);
+  const int lines = std::max(a.ied - a.isd, a.jed - a.jsd) + 1;
+  const dim3 ge((unsigned)((lines * 10 + 127) / 128), g.y, 2);
+  const bool edges = a.ew != NO_EDGE || a.ee != NO_EDGE || a.es != NO_EDGE || a.en != NO_EDGE;
   k_lin_inner<<<g, 128, 0, s>>>(a, tr);
+  if (edges) k_lin_edges<<<ge, 128, 0, s>>>(a, tr, 0);
   k_lin_mid<<<g, 128, 0, s>>>(a, tr.qc1, tr.qc2, tr.fx2, tr.fy2, tr.qi, tr.qj);
   k_lin_outer<<<g, 128, 0, s>>>(a, tr);
+  if (edges) k_lin_edges<<<ge, 128, 0, s>>>(a, tr, 1);
   FV3G_CUDA(cudaGetLastError());
   return 0;
 }

@@ -360,3 +360,21 @@ def test_c96_map1_ppm_kord4_adjoint_dot_product(cuda):
                     -1, 4)
     lhs, rhs = float((q2t[:, 0] * w).sum()), float((q1_ad[:, 0] * dq).sum())
     assert abs(lhs - rhs) <= DOT_TOL * abs(lhs), (lhs, rhs)
+
+
+@pytest.mark.parametrize("hord", [1, 5, 8])
+@pytest.mark.parametrize("n", [12, 13, 29])
+def test_face_weights_beside_the_edges_dot_product(cuda, n, hord):
+    """Closed-form face weights away from the cube-face edges, one-sided ones beside them: on the smallest tiles
+    (where few ordinary faces lie between the edges) and across a partial CTA tile, the adjoint assembled from
+    them is the transpose of the tangent-linear kernel, with clipped tracers (flat cells: exact ties)."""
+    d = _inputs(S.make_problem(n, 2, 2, seed=n, cmax=0.9), t=2, k=1, iq=1)
+    rng = np.random.default_rng(n)
+    dq = rng.standard_normal(d["q"].shape)
+    wx, wy = rng.standard_normal((n, n + 1)), rng.standard_normal((n + 1, n))
+    _, fxt, _, fyt = _tl(d, dq, hord)
+    q_ad = np.zeros_like(d["q"])
+    _ad(d, q_ad, wx, wy, hord)
+    lhs = float((fxt * wx).sum() + (fyt * wy).sum())
+    scale = float(np.abs(fxt * wx).sum() + np.abs(fyt * wy).sum())  # the sum's own magnitude
+    assert abs(lhs - float((q_ad * dq).sum())) <= DOT_TOL * scale
