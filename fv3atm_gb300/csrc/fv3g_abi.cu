@@ -123,6 +123,7 @@ struct fv3g_state {
   void* cx = nullptr; void* cy = nullptr; void* mfx = nullptr; void* mfy = nullptr;  // inputs (unscaled)
   void* cxs = nullptr; void* cys = nullptr; void* mfxs = nullptr; void* mfys = nullptr;  // scaled copies
   void* xfx = nullptr; void* yfx = nullptr;
+  void* lev = nullptr; void* ew = nullptr;  // FP64: the marching substep's per-level planes and edge weights (AdvArgs)
   void* dp_eul = nullptr;
   void* area = nullptr; void* rarea = nullptr; void* dxa = nullptr; void* dya = nullptr;
   void* dx = nullptr; void* dy = nullptr; void* sin4 = nullptr;
@@ -252,6 +253,11 @@ AdvArgs<T> adv_args(fv3g_state* st, int src, int dst, int dp_in, int dp_out) {
   a.mfy = (const T*)st->mfys;
   a.dp1 = (const T*)st->dp[dp_in];
   a.dp2 = (T*)st->dp[dp_out];
+  if (st->lev) {
+    T** const planes[STREAM_LEVEL_PLANES] = {&a.cx1, &a.cx2, &a.cy1, &a.cy2, &a.rrx, &a.rry, &a.dpa, &a.ub};
+    for (int i = 0; i < STREAM_LEVEL_PLANES; ++i) *planes[i] = (T*)st->lev + (long long)i * st->plane * st->npz * st->nt;
+    a.ew = (T*)st->ew;
+  }
   a.sFk = st->plane;
   a.sFt = st->plane * st->npz;
   a.area = (const T*)st->area;
@@ -402,6 +408,8 @@ int substeps_t(fv3g_state* st, int nsplt, int g0, int ng, cudaStream_t s, int k0
       a.cx += lo; a.cy += lo; a.xfx += lo; a.yfx += lo; a.mfx += lo; a.mfy += lo;
       a.dp1 += lo;
       a.dp2 += lo;
+      if (st->lev)
+        for (T** p : {&a.cx1, &a.cx2, &a.cy1, &a.cy2, &a.rrx, &a.rry, &a.dpa, &a.ub}) *p += lo;
       a.npz = nk;
     }
     a.nq = ng;
@@ -416,7 +424,7 @@ int substeps_t(fv3g_state* st, int nsplt, int g0, int ng, cudaStream_t s, int k0
                                      st->pg, st->n, s));
       CHECK(mark(st, K_HALO, s));
     }
-    CHECK(launch_substep<T>(a, st->d.hord, false, warps, s));
+    CHECK(launch_substep<T>(a, st->d.hord, false, warps, s, it == 0));
     const bool damp = it == 0 && st->d.trdm > 1e-4;  // upstream damps the first substep only
     if (damp) {
       a.del6_u = (const T*)st->del6u;
@@ -427,9 +435,10 @@ int substeps_t(fv3g_state* st, int nsplt, int g0, int ng, cudaStream_t s, int k0
       CHECK(launch_damp<T>(a, false, s));
     }
     {
+      // FP32: the interior and the edge-ring CTAs; FP64: the level planes and the march
       const BlockMap bm = block_map(a.is, a.ie, a.js, a.je, a.npx, a.npy, a.nested);
       const int nint = bm.nbxi * bm.nbyi;
-      CHECK(mark(st, K_SUBSTEP, s, (nint > 0) + (bm.nbx * bm.nby > nint) + (damp ? 1 : 0)));
+      CHECK(mark(st, K_SUBSTEP, s, (st->fp64 ? 2 : (nint > 0) + (bm.nbx * bm.nby > nint)) + (damp ? 1 : 0)));
     }
     if (st->cube && st->eflux != nullptr) {
       CHECK(launch_edge_fix<T>(a, st->n, s));
@@ -696,7 +705,7 @@ int lin_forward(fv3g_state* st, int q_split, cudaStream_t s, CallBufs& B, LinSte
     a.dp2 = L.dp[it + 1];
     a.eflux = nullptr;
     a.warps_ring = std::min(a.warps_ring, st->nq);
-    CHECK(launch_substep<double>(a, st->d.hord, false, warps, s));
+    CHECK(launch_substep<double>(a, st->d.hord, false, warps, s, it == 0));
   }
   if (L.nsplt > 0) st->last_nsplt = L.nsplt;
   // the linearised substep's arguments and buffers
@@ -879,6 +888,8 @@ int fv3g_state_create(const fv3g_state_desc* desc, fv3g_state** out) {
   for (void** m : metrics)
     if (!rc) rc = dalloc(st, m, P * nt);
   if (!rc) rc = dalloc(st, &st->sin4, P * nt * 4);
+  if (!rc && st->fp64) rc = dalloc(st, &st->lev, fb * STREAM_LEVEL_PLANES);
+  if (!rc && st->fp64) rc = dalloc(st, &st->ew, st->esz * nt * (size_t)st->pg.rows * 8);
   if (!rc && st->cube && d.edge_sync)
     rc = dalloc(st, &st->eflux, st->esz * 6 * 4 * (size_t)d.npz * d.nq * d.n);
   if (!rc) rc = dalloc(st, (void**)&st->ak, sizeof(double) * (KMAX + 1));

@@ -251,12 +251,65 @@ int prepare_kernels() {
     prepare_substep_hord<1>(err);
     prepare_substep_hord<5>(err);
     prepare_substep_hord<8>(err);
+    prepare_stream_h<1>(err);
+    prepare_stream_h<5>(err);
+    prepare_stream_h<8>(err);
   });
   return err == cudaSuccess ? 0 : cuda_error(err, "cudaFuncSetAttribute(advection kernels)");
 }
 
+// Per-level planes of the marching FP64 substep, shared by the level's tracers
+// (AdvArgs::cx1 .. ew): those of the Courant numbers and area fluxes in a step's
+// first substep, and the thickness update dp2 with 2 dp1/rarea and rarea/(2 dp2)
+// (the flux averages' halves) in every one.  Bound by HBM (about 20 planes moved
+// per level, once for all tracers).
+template <bool FIRST>
+__global__ void __launch_bounds__(256) k_level(const AdvArgs<double> a) {
+  const PlaneGeom& pg = a.pg;
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  const int jr = e / pg.pitch, ic = e - jr * pg.pitch;
+  if (jr >= pg.rows) return;
+  const int i = pg.isd + ic, j = pg.jsd + jr;
+  const long long p = (long long)blockIdx.z * a.sFt + blockIdx.y * a.sFk + e, pm = (long long)blockIdx.z * a.sMt + e;
+  if (FIRST) {
+    if (blockIdx.y == 0 && ic < 2 && !a.nested) {  // one thread per row and x edge
+      const double* d = a.dxa + (long long)blockIdx.z * a.sMt + (long long)jr * pg.pitch;
+      const int ex = ic == 0 ? 1 : a.npx;  // first cell beyond the edge face
+      double* w = a.ew + (((long long)blockIdx.z * pg.rows + jr) * 2 + ic) * 4;
+      double v[4];
+      for (int c = 0; c < 4; ++c) v[c] = d[min(max(ex - 2 + c - pg.isd, 0), pg.pitch - 1)];
+      w[0] = v[1] / (v[1] + v[0]);
+      w[1] = v[2] / (v[2] + v[3]);
+    }
+    auto face = [p](double c, double* w1, double* w2) {
+      const double m = fabs(c), w = 1.0 - m, v = m * w;
+      w1[p] = w;
+      w2[p] = ((__double2hiint(w) < 0) == (c > 0.0)) ? -fabs(v) : fabs(v);
+    };
+    face(a.cx[p], a.cx1, a.cx2);
+    face(a.cy[p], a.cy1, a.cy2);
+    if (i >= a.is && i <= a.ie) a.rrx[p] = 1.0 / (a.area[pm] + a.xfx[p] - a.xfx[p + 1]);
+    if (j >= a.js && j <= a.je) a.rry[p] = 1.0 / (a.area[pm] + a.yfx[p] - a.yfx[p + pg.pitch]);
+  }
+  if (i < a.is || i > a.ie || j < a.js || j > a.je) return;
+  const double d1 = a.dp1[p], ra = a.rarea[pm];
+  const double d2 = d1 + (a.mfx[p] - a.mfx[p + 1] + a.mfy[p] - a.mfy[p + pg.pitch]) * ra;
+  a.dpa[p] = 2.0 * (d1 / ra);
+  a.ub[p] = 0.5 * (ra / d2);
+  if (a.dp2 != nullptr) a.dp2[p] = d2;
+  if (!(d2 > 0.0)) raise_error(a.err, FV3G_E_DELP);
+}
+
+static int launch_level(const AdvArgs<double>& a, bool first, cudaStream_t s) {
+  const dim3 grid((unsigned)((a.pg.plane() + 255) / 256), a.npz, adv_tiles(a));
+  if (first) k_level<true><<<grid, 256, 0, s>>>(a);
+  else k_level<false><<<grid, 256, 0, s>>>(a);
+  FV3G_CUDA(cudaGetLastError());
+  return 0;
+}
+
 template <typename T>
-int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cudaStream_t s) {
+int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cudaStream_t s, bool first) {
   {
     int prc = prepare_kernels();
     if (prc) return prc;
@@ -264,6 +317,19 @@ int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cud
   if (hord == 1 && !(a.lim_fac > 0.0)) return set_error(FV3G_E_ARG, "hord 1 needs lim_fac > 0 (got %g)", a.lim_fac);
   if constexpr (std::is_same<T, float>::value) {
     if (a.pairs && hord == 8 && !flux_mode) return launch_substep_pair(a, warps, s);
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (!flux_mode && (hord == 8 || hord == 5 || hord == 1)) {
+      const int mw = substep_max_warps((int)sizeof(T));
+      if (warps < 1 || warps > mw || a.warps_ring < 0 || a.warps_ring > mw)
+        return set_error(FV3G_E_ARG,
+                         "this precision supports 1..%d advection warps per CTA and 1..%d per edge-ring CTA (got %d, %d)",
+                         mw, mw, warps, a.warps_ring);
+      const int rc = launch_level(a, first, s);
+      if (rc) return rc;
+      return hord == 8 ? launch_stream_h<8>(a, warps, s)
+                       : hord == 5 ? launch_stream_h<5>(a, warps, s) : launch_stream_h<1>(a, warps, s);
+    }
   }
   switch (hord) {
     case 8: return launch_substep_hord<T, 8>(a, flux_mode, warps, s);
@@ -372,7 +438,7 @@ int launch_max_courant(const T* cx, const T* cy, long long sFt, long long sFk, P
 }
 
 #define FV3G_INST(T)                                                                                          \
-  template int launch_substep<T>(const AdvArgs<T>&, int, bool, int, cudaStream_t);                          \
+  template int launch_substep<T>(const AdvArgs<T>&, int, bool, int, cudaStream_t, bool);                    \
   template int launch_edge_fix<T>(const AdvArgs<T>&, int, cudaStream_t);                                     \
   template int launch_cube_halo<T>(T*, long long, long long, int, PlaneGeom, int, const Topo&, cudaStream_t, int,  \
                                    long long);                                                                 \

@@ -243,7 +243,7 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
   const PlaneGeom pg = plane_for(bd);
   const size_t P = (size_t)pg.plane();
   const size_t nqp = (size_t)nq * npz;
-  CHECK(g_ctx.begin(padded(P * nqp, 8) * 2 + padded(P * npz, 8) * 9 + padded(P, 8) * 14 + 256 +
+  CHECK(g_ctx.begin(padded(P * nqp, 8) * 2 + padded(P * npz, 8) * 17 + padded(P, 8) * 14 + padded((size_t)pg.rows * 8, 8) + 256 +
                     (nest ? 2 * padded(nl.cells * nqp, 8) + 8 * 256 : 0)));
   cudaStream_t s = g_ctx.stream;
   double* qa = g_ctx.take<double>(P * nqp);
@@ -252,6 +252,13 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
   double *dcx = g_ctx.take<double>(P * npz), *dcy = g_ctx.take<double>(P * npz);
   double *dmx = g_ctx.take<double>(P * npz), *dmy = g_ctx.take<double>(P * npz);
   double *dxf = g_ctx.take<double>(P * npz), *dyf = g_ctx.take<double>(P * npz);
+  double* lev[STREAM_LEVEL_PLANES];  // the marching substep's per-level planes
+  for (double*& l : lev) l = g_ctx.take<double>(P * npz);
+  auto level_planes = [&](AdvArgs<double>& a, long long ko) {
+    double** const planes[STREAM_LEVEL_PLANES] = {&a.cx1, &a.cx2, &a.cy1, &a.cy2, &a.rrx, &a.rry, &a.dpa, &a.ub};
+    for (int i = 0; i < STREAM_LEVEL_PLANES; ++i) *planes[i] = lev[i] + ko;
+  };
+  double* ew = g_ctx.take<double>((size_t)pg.rows * 8);
   double *ddx = g_ctx.take<double>(P), *ddy = g_ctx.take<double>(P), *ddxa = g_ctx.take<double>(P);
   double *ddya = g_ctx.take<double>(P), *dar = g_ctx.take<double>(P), *drar = g_ctx.take<double>(P);
   double* dsin = g_ctx.take<double>(4 * P);
@@ -338,6 +345,8 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
         a.sQk = PL; a.sQq = PL * npz; a.sQt = 0;
         a.cx = dcx + ko; a.cy = dcy + ko; a.xfx = dxf + ko; a.yfx = dyf + ko; a.mfx = dmx + ko; a.mfy = dmy + ko;
         a.dp1 = dpb[dpi] + ko; a.dp2 = dpb[dpo] + ko;
+        level_planes(a, ko);
+        a.ew = ew;
         a.sFk = PL; a.sFt = 0;
         a.area = dar; a.rarea = drar; a.dxa = ddxa; a.dya = ddya; a.sMt = 0;
         a.pg = pg;
@@ -348,7 +357,7 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
         a.nested = grid->nested;
         a.cube = 0;
         a.lim_fac = lim_fac;
-        CHECK(launch_substep<double>(a, hord, false, std::min(nq, 4), s));
+        CHECK(launch_substep<double>(a, hord, false, std::min(nq, 4), s, it == 0));
         if (damping && it == 0) {
           a.del6_u = d6u;
           a.del6_v = d6v;
@@ -429,6 +438,8 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
     a.sQk = (long long)P; a.sQq = (long long)P * npz; a.sQt = 0;
     a.cx = dcx; a.cy = dcy; a.xfx = dxf; a.yfx = dyf; a.mfx = dmx; a.mfy = dmy;
     a.dp1 = dpb[dpi]; a.dp2 = dpb[dpo];
+    level_planes(a, 0);
+    a.ew = ew;
     a.sFk = (long long)P; a.sFt = 0;
     a.area = dar; a.rarea = drar; a.dxa = ddxa; a.dya = ddya; a.sMt = 0;
     a.pg = pg;
@@ -439,7 +450,7 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
     a.nested = grid->nested;
     a.cube = 0;
     a.lim_fac = lim_fac;
-    CHECK(launch_substep<double>(a, hord, false, std::min(nq, 4), s));
+    CHECK(launch_substep<double>(a, hord, false, std::min(nq, 4), s, it == 0));
     if (damping && it == 0) {
       a.del6_u = d6u;
       a.del6_v = d6v;

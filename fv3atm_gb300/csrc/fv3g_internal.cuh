@@ -42,6 +42,10 @@ struct Topo {
 // kernel is capped at 128 registers so that two 8-warp CTAs fit an SM.
 __host__ __device__ constexpr int ring_max_warps(int element_bytes) { return element_bytes == 4 ? 8 : 10; }
 
+// Widest advection CTA (warps) that a state of this element size accepts; the
+// marching FP64 substep takes the width as the most tracers of a CTA.
+__host__ __device__ constexpr int substep_max_warps(int element_bytes) { return element_bytes == 4 ? 10 : 6; }
+
 struct PlaneGeom {
   int pitch;  // elements per row
   int rows;   // rows per plane
@@ -97,6 +101,13 @@ struct AdvArgs {
   int nord;
   int damp_mass;    // 1: field q, flux weighted by damp times the face mean of dp1; 0: field damp q
   int* err;         // optional sticky error word: FV3G_E_DELP when a compute cell's dp2 is not positive
+  // FP64 marching substep (fv3g_stream.cuh): per-level planes that launch_level forms.  Once per step, from the
+  // Courant numbers and area fluxes: w1 = 1 - |c| and w2 = |c| w1 of the x and y faces (w2 with the sign of w1 where
+  // c > 0, else the other sign), 1/ra_x, 1/ra_y; every substep: 2 dp1/rarea and rarea/(2 dp2)
+  T *cx1, *cx2, *cy1, *cy2, *rrx, *rry, *dpa, *ub;
+  // [tile][plane row][west, east][4]: the weights d(e-1)/(d(e-1)+d(e-2)), d(e)/(d(e)+d(e+1)) of the one-sided edge
+  // value at the tile's x edges (d = dxa along the row, e the cell beyond the edge face); once per step
+  T* ew;
   int pairs;        // FP32, hord 8: advance the tracers two per warp (k_substep_pair)
   int ntiles;       // tiles the launches cover (0: 6 for the cube, else 1)
 };
@@ -248,6 +259,13 @@ int launch_substep_tl_hord(const AdvArgs<Dual<double>>& a, cudaStream_t s);
 template <int HORD>
 void prepare_substep_hord(cudaError_t& err);
 
+// Marching FP64 substep kernels, one translation unit per hord (fv3g_stream_h*.cu)
+constexpr int STREAM_LEVEL_PLANES = 8;  // per-level planes of AdvArgs (cx1 .. ub)
+template <int HORD>
+int launch_stream_h(const AdvArgs<double>& a, int warps, cudaStream_t s);
+template <int HORD>
+void prepare_stream_h(cudaError_t& err);
+
 // Tracer damping (fv3g_damp.cu): adds the deln_flux fluxes of a substep's
 // input q_in (a.damp, a.nord) to the fluxes (flux mode) or to q_out and the
 // tile-edge fluxes; runs after the substep kernel on the same stream.
@@ -265,8 +283,10 @@ int launch_substep_tl(const AdvArgs<Dual<double>>& a, int hord, cudaStream_t s);
 template <typename T>
 int launch_cube_halo(T* q, long long sQt, long long splane, int nplanes, PlaneGeom pg, int n, const Topo& topo,
                      cudaStream_t s, int nlev = 0, long long sQq = 0);  // nlev > 0: planes of nlev levels, sQq apart
+// flux_mode: fv_tp_2d's fluxes; else the substep's update, which for FP64 needs the planes a.cx1 .. a.ew; first: the
+// step's first substep, which forms those that the substeps share.
 template <typename T>
-int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cudaStream_t s);
+int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cudaStream_t s, bool first = true);
 int launch_substep_pair(const AdvArgs<float>& a, int warps, cudaStream_t s);
 constexpr int PAIR_WIDTH_MAX = 12;  // warps (tracer pairs) per CTA of the paired substep
 template <typename T>

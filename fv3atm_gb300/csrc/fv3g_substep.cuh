@@ -23,6 +23,8 @@
 // the neighbouring tiles of the cube (or read from the caller's halo), and
 // the cube-corner blocks are filled by the rotation of copy_corners at load.
 //
+// FP32 states' substep, and the flux mode of the FP64 and tangent-linear
+// fv_tp_2d entries; the FP64 substep is the march of fv3g_stream.cuh.
 // This header holds the kernel templates; fv3g_substep_h{1,5,8}.cu instantiate
 // them once per hord, so the three compile in parallel.
 #pragma once
@@ -814,10 +816,11 @@ static void set_attrs_tl(cudaError_t& err) {
     if (e != cudaSuccess && err == cudaSuccess) err = e;
 }
 
+// FP32: the update; FP64: fv_tp_2d's fluxes (its update is the march of fv3g_stream.cuh)
 template <typename T, int HORD>
 static void set_attrs(cudaError_t& err) {
-  cudaError_t es[] = {set_smem_attr<T, HORD, false, false>(), set_smem_attr<T, HORD, false, true>(),
-                      set_smem_attr<T, HORD, true, false>(), set_smem_attr<T, HORD, true, true>()};
+  constexpr bool FLUXES = sizeof(T) != 4;
+  cudaError_t es[] = {set_smem_attr<T, HORD, FLUXES, false>(), set_smem_attr<T, HORD, FLUXES, true>()};
   for (cudaError_t e : es)
     if (e != cudaSuccess && err == cudaSuccess) err = e;
 }
@@ -829,7 +832,9 @@ int launch_substep_hord(const AdvArgs<T>& a, bool flux_mode, int warps, cudaStre
     return set_error(FV3G_E_ARG,
                      "this precision supports 1..%d advection warps per CTA and 1..%d per edge-ring CTA (got %d, %d)",
                      mw, mr, warps, a.warps_ring);
-  return flux_mode ? launch_one<T, HORD, true>(a, warps, s) : launch_one<T, HORD, false>(a, warps, s);
+  constexpr bool FLUXES = sizeof(T) != 4;
+  if (flux_mode != FLUXES) return set_error(FV3G_E_UNSUPPORTED, "windowed advection: FP32 update or FP64 fluxes");
+  return launch_one<T, HORD, FLUXES>(a, warps, s);
 }
 
 template <int HORD>
