@@ -9,6 +9,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "fv3g_fp64.cuh"
 #include "fv3g_stencil.cuh"
 
 namespace fv3g {
@@ -278,8 +279,11 @@ __global__ void __launch_bounds__(256) k_level(const AdvArgs<double> a) {
       double* w = a.ew + (((long long)blockIdx.z * pg.rows + jr) * 2 + ic) * 4;
       double v[4];
       for (int c = 0; c < 4; ++c) v[c] = d[min(max(ex - 2 + c - pg.isd, 0), pg.pitch - 1)];
-      w[0] = v[1] / (v[1] + v[0]);
-      w[1] = v[2] / (v[2] + v[3]);
+      const double wl = v[1] / (v[1] + v[0]), wr = v[2] / (v[2] + v[3]);
+      w[0] = -0.5 * wl;
+      w[1] = 0.5 + 0.5 * wl;
+      w[2] = 0.5 + 0.5 * wr;
+      w[3] = -0.5 * wr;
     }
     auto face = [p](double c, double* w1, double* w2) {
       const double m = fabs(c), w = 1.0 - m, v = m * w;
@@ -288,14 +292,14 @@ __global__ void __launch_bounds__(256) k_level(const AdvArgs<double> a) {
     };
     face(a.cx[p], a.cx1, a.cx2);
     face(a.cy[p], a.cy1, a.cy2);
-    if (i >= a.is && i <= a.ie) a.rrx[p] = 1.0 / (a.area[pm] + a.xfx[p] - a.xfx[p + 1]);
-    if (j >= a.js && j <= a.je) a.rry[p] = 1.0 / (a.area[pm] + a.yfx[p] - a.yfx[p + pg.pitch]);
+    if (i >= a.is && i <= a.ie) a.rrx[p] = fast_rcp(a.area[pm] + a.xfx[p] - a.xfx[p + 1]);
+    if (j >= a.js && j <= a.je) a.rry[p] = fast_rcp(a.area[pm] + a.yfx[p] - a.yfx[p + pg.pitch]);
   }
   if (i < a.is || i > a.ie || j < a.js || j > a.je) return;
   const double d1 = a.dp1[p], ra = a.rarea[pm];
   const double d2 = d1 + (a.mfx[p] - a.mfx[p + 1] + a.mfy[p] - a.mfy[p + pg.pitch]) * ra;
-  a.dpa[p] = 2.0 * (d1 / ra);
-  a.ub[p] = 0.5 * (ra / d2);
+  a.dpa[p] = 2.0 * fast_div(d1, ra);
+  a.ub[p] = 0.5 * fast_div(ra, d2);
   if (a.dp2 != nullptr) a.dp2[p] = d2;
   if (!(d2 > 0.0)) raise_error(a.err, FV3G_E_DELP);
 }

@@ -105,8 +105,8 @@ struct AdvArgs {
   // Courant numbers and area fluxes: w1 = 1 - |c| and w2 = |c| w1 of the x and y faces (w2 with the sign of w1 where
   // c > 0, else the other sign), 1/ra_x, 1/ra_y; every substep: 2 dp1/rarea and rarea/(2 dp2)
   T *cx1, *cx2, *cy1, *cy2, *rrx, *rry, *dpa, *ub;
-  // [tile][plane row][west, east][4]: the weights d(e-1)/(d(e-1)+d(e-2)), d(e)/(d(e)+d(e+1)) of the one-sided edge
-  // value at the tile's x edges (d = dxa along the row, e the cell beyond the edge face); once per step
+  // [tile][plane row][west, east][4]: the one-sided edge value at the tile's x edges as a linear form of the cells
+  // e-2..e+1 of the row (e the cell beyond the edge face; weights from dxa); once per step
   T* ew;
   int pairs;        // FP32, hord 8: advance the tracers two per warp (k_substep_pair)
   int ntiles;       // tiles the launches cover (0: 6 for the cube, else 1)

@@ -2,8 +2,9 @@
 // with the cs_profile reconstruction of fv_mapz.F90, GFDL_atmos_cubed_sphere,
 // absent submodule .gitmodules:1-4).
 //
-// Two kernels share the schemes of fv3g_profile.cuh:
-//   * k_remap_warp, the batched and drop-in remap: one warp per column, lane l
+// Two kernels share the schemes of fv3g_profile.cuh (FP64 fields' remap is
+// fv3g_remap64.cu):
+//   * k_remap_warp, the FP32 remap: one warp per column, lane l
 //     owning interfaces / layers l*NPL .. l*NPL+NPL-1, the column's constants
 //     (interface pressures, overlap schedule, LU factors of the interface
 //     system) in registers for all its fields, the recurrences as warp scans
@@ -416,8 +417,9 @@ __device__ __forceinline__ T affine_enter_bwd(T al, T be, int lane) {
   return __shfl_down_sync(0xffffffffu, be, 1);
 }
 
-template <typename T, int KORD, int NPL>
-__global__ void __launch_bounds__(32 * RCOL, sizeof(T) == 4 ? 2 : 1) k_remap_warp(const RemapArgs<T> a) {
+template <typename T, int KORD, int NPL>  // T: float (FP64 columns: k_remap64)
+__global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> a) {
+  static_assert(Single<T>::value, "FP32 columns");
   constexpr int RING = ring_slots<T>(), RP = ring_pitch<T, NPL>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -744,7 +746,7 @@ __global__ void __launch_bounds__(32 * RCOL, sizeof(T) == 4 ? 2 : 1) k_remap_war
         }
       }
     }
-    if (Single<T>::value) {
+    {
       // FP32 fields: cumulative source mass in float-float at every source
       // interface (layer masses q*dp are exact as float-float products), so a
       // target layer's mass is a difference of two cumulative values and the
@@ -788,7 +790,7 @@ __global__ void __launch_bounds__(32 * RCOL, sizeof(T) == 4 ? 2 : 1) k_remap_war
     // ------------------------------------------------------- integration
 #pragma unroll
     for (int h = 0; h < FP; ++h) {
-      if (Single<T>::value) {
+      {
         // cumulative mass at this lane's target interfaces; the last one is the
         // next lane's first (32 NPL > kn, so lane 31's last is never used)
         FF cm[NPL + 1];
@@ -822,26 +824,6 @@ __global__ void __launch_bounds__(32 * RCOL, sizeof(T) == 4 ? 2 : 1) k_remap_war
           const float qq = fmaf(fmaf(-q0, d, mm), r, q0);
           if (store[h] && t < kn) q2[h][(long long)t * a.sQk] = T(qq);
         }
-      } else {
-#pragma unroll
-        for (int j = 0; j < NPL; ++j) {
-          const int t = u0 + j;
-          const int Lt = Ls[j], Lb = Ls[j + 1];
-          const T Xt = Xs[j], Xb = Xs[j + 1];
-          const bool inside = (Lb == Lt) || (Lb == Lt + 1 && Xb == T(0));
-          const int it = pk<T>(Lt), ib_ = pk<T>(Lb);
-          const T qt = Q[h][it], dpt = S.dp[it];
-          const T pm1 = pmean(S.pl[h][it], S.pr[h][it], S.p6[h][it], Xt, (inside && Lb == Lt) ? Xb : T(1));
-          const T vin = (Xt == T(0) && (Lb == Lt + 1 || Xb == T(1))) ? qt : pm1;
-          T mass = Xt == T(0) ? qt * dpt : (dpt * (T(1) - Xt)) * pm1;
-          for (int mm = Lt + 1; mm < Lb; ++mm) mass = mass + Q[h][pk<T>(mm)] * S.dp[pk<T>(mm)];
-          const T qb_ = Q[h][ib_], dpb = S.dp[ib_];
-          const T pm2 = pmean(S.pl[h][ib_], S.pr[h][ib_], S.p6[h][ib_], T(0), Xb);
-          const T bot = Xb >= T(1) ? qb_ * (dpb * Xb) : (Xb > T(0) ? (dpb * Xb) * pm2 : T(0));
-          mass = mass + bot;
-          const T out = inside ? vin : mass * rdpk[j];
-          if (store[h] && t < kn) q2[h][(long long)t * a.sQk] = out;
-        }
       }
     }
   }
@@ -859,9 +841,8 @@ int prepare_remap_kernels() {
   static std::once_flag once;
   static cudaError_t err = cudaSuccess;
   std::call_once(once, [] {
-    cudaError_t es[] = {set_remap_attr<float, 9, 4>(),  set_remap_attr<float, 9, 5>(),  set_remap_attr<float, 4, 4>(),
-                        set_remap_attr<float, 4, 5>(),  set_remap_attr<double, 9, 4>(), set_remap_attr<double, 9, 5>(),
-                        set_remap_attr<double, 4, 4>(), set_remap_attr<double, 4, 5>()};
+    cudaError_t es[] = {set_remap_attr<float, 9, 4>(), set_remap_attr<float, 9, 5>(), set_remap_attr<float, 4, 4>(),
+                        set_remap_attr<float, 4, 5>(), prepare_remap64()};
     for (cudaError_t e : es)
       if (e != cudaSuccess && err == cudaSuccess) err = e;
   });
@@ -902,6 +883,8 @@ int launch_remap(const RemapArgs<T>& a, int kord, cudaStream_t s) {
     const unsigned nb = (unsigned)((a.ncol + 127) / 128);
     if (kord == 9) k_remap_scratch<T, 9><<<nb, 128, 0, s>>>(a);
     else k_remap_scratch<T, 4><<<nb, 128, 0, s>>>(a);
+  } else if constexpr (std::is_same<T, double>::value) {
+    FV3G_CUDA(launch_remap64(a, kord, s));
   } else {
     const cudaError_t e = kord == 9 ? launch_warp_form<T, 9>(a, s) : launch_warp_form<T, 4>(a, s);
     FV3G_CUDA(e);

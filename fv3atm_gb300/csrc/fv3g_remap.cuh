@@ -46,6 +46,9 @@ size_t remap_scratch_bytes(long long ncol, size_t elem_bytes);
 bool remap_col_applies(const RemapArgs<float>& a, int kord);
 cudaError_t launch_remap_col(const RemapArgs<float>& a, cudaStream_t s);  // scratch + schedule of the scratch kernel
 int prepare_remap_kernels();
+// the FP64 warp-per-column kernel (fv3g_remap64.cu)
+cudaError_t prepare_remap64();
+cudaError_t launch_remap64(const RemapArgs<double>& a, int kord, cudaStream_t s);
 int launch_remap_tl(const RemapArgs<Dual<double>>& a, int kord, cudaStream_t s);
 // interface pressures of the columns of a field kind (cells, u or v faces) for the remap of extra fields
 template <typename T>

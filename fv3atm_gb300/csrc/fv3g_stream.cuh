@@ -33,14 +33,15 @@
 // which instruction issue bounds, keep the windowed kernel: this march took 6.1 ms
 // there against 6.0 at 6 x C192 L127 x 9 tracers, and 11.2 against 11.1 at 6 x C384
 // L64 x 16.  Measured FP64: a step of 6 x C192 L127 x 9 tracers, n_split 3, hord 8,
-// 460 -> 238 ms; 6 x C96 L64 x 4, 6 substeps, hord 5, 42.8 -> 37.2 ms; one C48 face,
-// 63 levels, one tracer, 0.79 -> 0.61 ms.
+// 460 -> 238 ms; 6 x C96 L64 x 4, 6 substeps, hord 5, 42.8 -> 37.2 ms; the substep of
+// the latter 3.7 -> 2.4 ms with one linear form for ordinary and one-sided interfaces
+// and no FP64 comparison left.
 #pragma once
 
 #include <algorithm>
 #include <type_traits>
 
-#include "fv3g_pair.cuh"
+#include "fv3g_fp64.cuh"
 #include "fv3g_stencil.cuh"
 
 namespace fv3g {
@@ -129,35 +130,6 @@ __device__ __forceinline__ Vec<NC> veast(const Vec<NC>& a) {
   return r;
 }
 
-// ------------------------------------------------------ scalar operations ---
-// FP64 bit patterns: |a| < |b|, the smaller magnitude, halves and doubles of
-// normal numbers, a > 0.
-__device__ __forceinline__ unsigned long long dbits(double a) { return (unsigned long long)__double_as_longlong(a); }
-__device__ __forceinline__ double mag_min(double a, double b) {  // of non-negative values
-  return dbits(a) < dbits(b) ? a : b;
-}
-// a 2^K for K = -2, -1, 1; a zero or of magnitude below 2^-1019 becomes zero
-template <int K>
-__device__ __forceinline__ double scale2(double a) {
-  const int hi = __double2hiint(a);
-  const bool ok = (hi & 0x7fffffff) >= 0x00400000;
-  return __hiloint2double(ok ? hi + K * 0x00100000 : 0, ok ? __double2loint(a) : 0);
-}
-// |a|, -a and a with the sign of b through the high word: as FP64 instructions they would take the FP64 pipe
-__device__ __forceinline__ double absv(double a) {
-  return __hiloint2double(__double2hiint(a) & 0x7fffffff, __double2loint(a));
-}
-__device__ __forceinline__ double negv(double a) {
-  return __hiloint2double(__double2hiint(a) ^ 0x80000000, __double2loint(a));
-}
-__device__ __forceinline__ double signed_as(double a, double b) {  // of a >= 0
-  return __hiloint2double(__double2hiint(a) | (__double2hiint(b) & 0x80000000), __double2loint(a));
-}
-__device__ __forceinline__ bool is_pos(double a) { return __double_as_longlong(a) > 0; }
-__device__ __forceinline__ bool opposite_signs(double a, double b) {
-  return (__double2hiint(a) ^ __double2hiint(b)) < 0 && (dbits(a) << 1) != 0 && (dbits(b) << 1) != 0;
-}
-
 // Monotonized central slopes in half increments: dm, |2 dm| and the sign; dp
 // and d are the differences to the cells before and after.
 template <int NC>
@@ -235,25 +207,14 @@ __device__ __forceinline__ Vec<NC> upwind(const FaceC<NC>& f, const Vec<NC>& xl,
 template <int HORD>
 __device__ __forceinline__ bool filter_pass(double lim, double nl, double br, double b0) {
   if (HORD == 1) return dbits(absv(lim * b0)) < dbits(absv(nl + br));
-  return opposite_signs(negv(nl), br);
+  return opp(negv(nl), br);
 }
 
-// a into the range of x0 and x1; FP64 by integer comparisons of order-preserving keys
-__device__ __forceinline__ long long dkey(double a) {
-  const long long k = __double_as_longlong(a);
-  return k ^ ((k >> 63) & 0x7fffffffffffffffLL);
-}
-__device__ __forceinline__ double clamp_between(double a, double x0, double x1) {
-  const bool up = dkey(x0) < dkey(x1);
-  const double lo = up ? x0 : x1, hi = up ? x1 : x0;
-  return dkey(a) < dkey(lo) ? lo : dkey(a) > dkey(hi) ? hi : a;
+// a linear form of four cells
+__device__ __forceinline__ double form4(const double* w, double x2, double x1, double x0, double x3) {
+  return fma(w[0], x2, fma(w[1], x1, fma(w[2], x0, w[3] * x3)));
 }
 
-// the edge value (mean of the two one-sided extrapolations) of edge e from
-// cells e-2..e+1 and the weights d(e-1)/(d(e-1)+d(e-2)), d(e)/(d(e)+d(e+1))
-__device__ __forceinline__ double edge_value(double x2, double x1, double x0, double x3, double wl, double wr) {
-  return double(0.5) * ((x1 + wl * (x1 - x2)) + (x0 - wr * (x3 - x0)));
-}
 // hord 8: raw deviations (of the cell before: rb, after: ra) of the interface
 // between x1 and x0 beside a cube-face edge e: kind 1 interface e-1, 2 the edge, 3
 // e+1; high: the tile lies below the edge.  x2, x3 the cells beyond x1 and x0, dm1
@@ -261,7 +222,7 @@ __device__ __forceinline__ double edge_value(double x2, double x1, double x0, do
 __device__ __forceinline__ void edge_raw8(int kind, bool high, double x2, double x1, double x0, double x3, double dm1, double dm0, const double* w, double& rb,
                                           double& ra) {
   if (kind == 2) {
-    const double a0 = clamp_between(edge_value(x2, x1, x0, x3, w[0], w[1]), x1, x0);
+    const double a0 = clamp_between(form4(w, x2, x1, x0, x3), x1, x0);
     rb = a0 - x1;
     ra = a0 - x0;
   } else if (kind == 1) {
@@ -281,26 +242,33 @@ __device__ __forceinline__ void edge_raw8(int kind, bool high, double x2, double
   }
 }
 
-// hord 1 / 5 interface between the second and third of four cells
+// hord 1 / 5 interface between the second and third of four cells, by kind: 0 the
+// fourth-order value, 1 and 3 the one-sided values beside a cube-face edge, 2 the
+// edge value with weights w.  One form with weights chosen by kind costs four FP64
+// instructions, as the fourth-order value alone does.
 __device__ __forceinline__ double interface4(double x2, double x1, double x0, double x3) {
-  return double(7.0 / 12.0) * (x1 + x0) - double(1.0 / 12.0) * (x2 + x3);
+  return (7.0 / 12.0) * (x1 + x0) - (1.0 / 12.0) * (x2 + x3);
 }
-// the same at a one-sided interface (kinds as above, 2: the edge)
-__device__ __forceinline__ double interface_edge(int kind, double x2, double x1, double x0, double x3, const double* w) {
-  if (kind == 1) return double(kD1) * x2 + double(kD2) * x1 + double(kD3) * x0;
-  if (kind == 3) return double(kD3) * x1 + double(kD2) * x0 + double(kD1) * x3;
-  return edge_value(x2, x1, x0, x3, w[0], w[1]);
+__device__ __forceinline__ double interface_edge(int kind, double x2, double x1, double x0, double x3,
+                                                 const double* w) {
+  double c[4];
+  c[0] = kind == 2 ? w[0] : kind == 1 ? kD1 : kind == 3 ? 0.0 : -1.0 / 12.0;
+  c[1] = kind == 2 ? w[1] : kind == 1 ? kD2 : kind == 3 ? kD3 : 7.0 / 12.0;
+  c[2] = kind == 2 ? w[2] : kind == 1 ? kD3 : kind == 3 ? kD2 : 7.0 / 12.0;
+  c[3] = kind == 2 ? w[3] : kind == 1 ? 0.0 : kind == 3 ? kD1 : -1.0 / 12.0;
+  return form4(c, x2, x1, x0, x3);
 }
 
-// cw84 with selects in place of branches (lanes beside an edge take different cases)
+// CW84 eq. 1.10 with selects: 3 |d (bl + br)| > d^2, d = br - bl, as 3 |bl + br| > |d|
 __device__ __forceinline__ void cw84_flat(double& bl, double& br) {
-  const double d = br - bl, t = 3.0 * d * (bl + br), d2 = d * d;
-  const bool flat = !opposite_signs(bl, br), big = dbits(absv(t)) > dbits(d2);
-  const bool lo = big && __double2hiint(t) < 0, hi = big && !lo;
-  const double nl = lo ? negv(scale2<1>(br)) : bl, nr = hi ? negv(scale2<1>(bl)) : br;
+  const double d = br - bl, s = bl + br;
+  const bool big = mag_less(absv(d), absv(3.0 * s)), down = (__double2hiint(d) ^ __double2hiint(s)) < 0;
+  const double nl = big && down ? negv(scale2<1>(br)) : bl, nr = big && !down ? negv(scale2<1>(bl)) : br;
+  const bool flat = !opp(bl, br);
   bl = flat ? 0.0 : nl;
   br = flat ? 0.0 : nr;
 }
+
 // What a y march meets at its next face (row-uniform): the interface kind (1:
 // e-1, 2: the cube-face edge e, 3: e+1, 0: none) and whether the cell it
 // completes takes CW84 (hord 8).  high: the edge is the tile's north one.
@@ -328,7 +296,7 @@ struct YLine {
   }
   template <bool SPEC>
   __device__ __forceinline__ V step(const V& x, const FaceC<NC>& f, double lim, const RowSpec& rs,
-                                    const double (&dw)[NC][2]) {
+                                    const double (&dw)[NC][4]) {
     V nl, br, rn, b0;
     bool keep[NC];
     const V d = x - xc;
@@ -348,7 +316,7 @@ struct YLine {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           double l = rl[c], r = rr[c];
-          cw84(l, r);
+          cw84_flat(l, r);
           nl[c] = -l;
           br[c] = r;
         }
@@ -444,11 +412,9 @@ __device__ __forceinline__ Vec<NC> x_line(const Vec<NC>& x, const FaceC<NC>& f, 
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const double x2 = c ? xm[c ? c - 1 : 0] : xw;
-      al[c] = interface4(x2, xm[c], x[c], xp[c]);
-      if (EDGES && le.kind[c] != 0)
-        al[c] = interface_edge(le.kind[c], x2, xm[c], x[c], xp[c], dw + le.side * 4);
+      al[c] = EDGES ? interface_edge(le.kind[c], x2, xm[c], x[c], xp[c], dw + le.side * 4)
+                    : interface4(x2, xm[c], x[c], xp[c]);
     }
-    if (EDGES) __syncwarp();
     const V ae = veast(al);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -576,7 +542,7 @@ struct March {
     }
     // ---- y sweeps to face m-2: q_i(m-3) and the final y flux
     RowSpec rs{0, false, false};
-    double dw[NC][2];
+    double dw[NC][4];
     if (SPEC) {
       const int f = m - 1, cell = m - 2;  // window rows of the next interface and of the cell completed
       rs.kind = eS != NO_EDGE && f >= eS - 1 && f <= eS + 1 ? f - eS + 2
@@ -590,8 +556,11 @@ struct March {
           const int i = i0 - 3 + lane * NC + c, je = j0 - 3 + f;
           const double d2 = ld_field(dya, pg, i, je - 2), d1 = ld_field(dya, pg, i, je - 1), d0 = ld_field(dya, pg, i, je),
                   d3 = ld_field(dya, pg, i, je + 1);
-          dw[c][0] = d1 / (d1 + d2);
-          dw[c][1] = d0 / (d0 + d3);
+          const double wl = d1 / (d1 + d2), wr = d0 / (d0 + d3);
+          dw[c][0] = -0.5 * wl;
+          dw[c][1] = 0.5 + 0.5 * wl;
+          dw[c][2] = 0.5 + 0.5 * wr;
+          dw[c][3] = -0.5 * wr;
         }
       }
     }

@@ -41,3 +41,28 @@ def test_tracer_groups_do_not_change_results(cuda, warps):
         got.append(st.download("Q"))
         st.close()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("kord", [9, 4])
+@pytest.mark.parametrize("km,kn", [(1, 3), (2, 2), (3, 5), (4, 4), (31, 31), (32, 32), (63, 64), (64, 63), (95, 95), (96, 40),
+                                   (127, 127), (128, 128), (20, 100)])
+@pytest.mark.parametrize("iv", [0, 1, -1])
+def test_fp64_remap_matches_oracle(cuda, km, kn, kord, iv):
+    """The FP64 column remap at the level counts where its lanes' layers change, onto finer and coarser targets;
+    tracers with zeros and jumps (the positivity scaling), columns that straddle several source layers."""
+    rng = np.random.default_rng(100 * km + kn + kord)
+    ncol = 37
+    pe1 = np.cumsum(np.vstack([np.full((1, ncol), 100.0), rng.uniform(0.2, 2.0, (km, ncol))]), axis=0)
+    frac = np.sort(np.vstack([np.zeros((1, ncol)), rng.uniform(0.0, 1.0, (kn - 1, ncol)), np.ones((1, ncol))]), axis=0)
+    pe2 = pe1[:1] + frac * (pe1[-1:] - pe1[:1])
+    pe2[-1] = pe1[-1]
+    q = rng.uniform(-1.0, 1.0, (2, km, ncol))
+    q[0] = np.maximum(q[0], 0.0)
+    ref = np.stack([O.remap_columns(pe1, x, pe2, iv=iv, kord=kord, q_min=0.1 if iv == 1 else 0.0) for x in q])
+    got = np.zeros((2, kn, 1, ncol))
+    api.map_scalar_3d(km, np.ascontiguousarray(pe1[:, None]), np.ascontiguousarray(q[:, :, None]), None, kn,
+                      np.ascontiguousarray(pe2[:, None]), got, 1, ncol, 1, 1, 1, ncol, 1, 1, 2, iv, kord,
+                      0.1 if iv == 1 else 0.0)
+    ok = np.isfinite(ref)  # kord 9's interface system of two layers is singular: the oracle divides by zero there
+    assert ok.all() or (km == 2 and kord == 9)
+    assert rel_l2(got[:, :, 0][ok], ref[ok]) <= FP64_TOL
