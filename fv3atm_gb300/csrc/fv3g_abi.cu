@@ -717,6 +717,13 @@ int lin_forward(fv3g_state* st, int q_split, cudaStream_t s, CallBufs& B, LinSte
   a.mfx = (const double*)st->mfxs; a.mfy = (const double*)st->mfys;
   a.area = (const double*)st->area; a.rarea = (const double*)st->rarea;
   a.dxa = (const double*)st->dxa; a.dya = (const double*)st->dya;
+  {
+    const AdvArgs<double> f = adv_args<double>(st, 0, 0, 0, 0);  // the forward substeps' reciprocals
+    a.rrx = f.rrx;
+    a.rry = f.rry;
+  }
+  CHECK(B.take(&a.dr, L.fn));
+  CHECK(B.take(&a.r2, L.fn));
   double** tq[] = {&L.tr.qc1, &L.tr.qc2, &L.tr.qi, &L.tr.qj, &L.tr.fx2, &L.tr.fy2,
                    &L.w.a1, &L.w.a2, &L.w.ai, &L.w.aj, &L.w.gx, &L.w.gy, &L.w.fx2, &L.w.fy2};
   for (double** b : tq) CHECK(B.take(b, L.qn));
@@ -1101,7 +1108,15 @@ int fv3g_state_step_tl(fv3g_state* st, int q_split, int parts, const double* dq_
     FV3G_CUDA(cudaStreamSynchronize(s));
     return 0;
   }
-  // the remap on (value, tangent) planes: the production kernel's tangent-linear instance
+  if (st->d.kord == 4) {
+    FV3G_CUDA(cudaMemsetAsync(dq1, 0, sizeof(double) * L.qn, s));
+    CHECK(lin_remap_tl4(L.q[L.nsplt], dq0, L.dp[L.nsplt], st->ak, st->bk, dq1, st->pg, st->plane, st->n, st->nt, st->nq,
+                        st->npz, st->npz, st->d.iv, st->d.q_min, s));
+    CHECK(lin_user_copy(st, dq1, dq_out, true, s));
+    FV3G_CUDA(cudaStreamSynchronize(s));
+    return 0;
+  }
+  // kord 9: the remap on (value, tangent) planes, the scratch kernel's tangent-linear instance
   using D2 = Dual<double>;
   D2 *qd, *qo, *dpd, *scr;
   unsigned char* sched;

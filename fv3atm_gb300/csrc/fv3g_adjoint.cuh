@@ -39,7 +39,9 @@ struct LinArgs {
   // frozen inputs of the substep (per-level planes, scaled by 1/nsplt)
   const double *cx, *cy, *xfx, *yfx, *mfx, *mfy;  // mfx / mfy: the weights of the face fluxes (times 0.5)
   const double *ra_x, *ra_y;  // optional; else area + xfx(i) - xfx(i+1), area + yfx(j) - yfx(j+1)
-  const double *dp1, *dp2;  // layer thickness at the substep's start and end
+  const double *rrx, *rry;    // optional: 1/ra_x, 1/ra_y formed by the forward substeps (else divided here)
+  const double *dp1, *dp2;    // layer thickness at the substep's start and end
+  double *dr, *r2;            // six-tile state: work planes dp1/dp2 and rarea/dp2 (lin_trajectory forms them)
   const double *area, *rarea, *dxa, *dya;
 };
 
@@ -94,6 +96,11 @@ int lin_remap_ad(const double* q, const double* dp, const double* ak, const doub
 // q1_ad += J^T q2_ad.
 int lin_remap_ad_rows(const double* q1, const double* pe1, const double* pe2, const double* qs, const double* q2_ad,
                       double* q1_ad, int ncol, int km, int kn, int iv, int kord, cudaStream_t s);
+
+// Tangent-linear of the same remap (kord 4): dq2 = J dq at the trajectory q, interior cells.
+int lin_remap_tl4(const double* q, const double* dq, const double* dp, const double* ak, const double* bk, double* dq2,
+                  PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv, double q_min,
+                  cudaStream_t s);
 
 // (value, tangent) planes from value and tangent arrays (d may be null: zero
 // tangent), and the tangents back out

@@ -378,3 +378,64 @@ def test_face_weights_beside_the_edges_dot_product(cuda, n, hord):
     lhs = float((fxt * wx).sum() + (fyt * wy).sum())
     scale = float(np.abs(fxt * wx).sum() + np.abs(fyt * wy).sum())  # the sum's own magnitude
     assert abs(lhs - float((q_ad * dq).sum())) <= DOT_TOL * scale
+
+
+# ------------------------------------- closed-form derivatives of the kord-4 column
+def _clipped_columns(km, ni, seed):
+    """Columns with noise, plateaus at zero (exact ties, layers at the floor) and a linear stretch."""
+    pe1, pe2, q1, rng = _row(km=km, ni=ni, seed=seed)
+    q1 = np.where(rng.uniform(size=q1.shape) < 0.3, 0.0, q1)
+    q1[:, ::3] = np.linspace(1.0, 2.0, km)[:, None]
+    return pe1, pe2, np.ascontiguousarray(q1), rng
+
+
+@pytest.mark.parametrize("iv", [-2, -1, 0, 1])
+@pytest.mark.parametrize("km", [3, 4, 5, 6, 31, 127])
+def test_column_adjoint_closed_forms_dot_product(cuda, km, iv):
+    """The reverse column (closed-form derivatives) against the tangent-linear column on dual numbers, at the
+    level counts where the end layers meet and at the largest, with layers at the floor."""
+    pe1, pe2, q1, rng = _clipped_columns(km, 24, km)
+    ni = q1.shape[1]
+    dq, w = rng.standard_normal(q1.shape), rng.standard_normal((km, ni))
+    qs = rng.standard_normal(ni) if iv == -2 else None
+    q2t, q1_ad = np.zeros((km, 1, ni)), np.zeros((km, 1, ni))
+    api.map1_ppm_tl(km, pe1, q1[:, None, :].copy(), dq[:, None, :].copy(), qs, km, pe2, None, q2t, 1, ni, 1, 1, ni,
+                    1, 1, iv, 4)
+    api.map1_ppm_ad(km, pe1, q1[:, None, :].copy(), q1_ad, qs, km, pe2, w[:, None, :].copy(), 1, ni, 1, 1, ni, 1, 1,
+                    iv, 4)
+    lhs, scale = float((q2t[:, 0] * w).sum()), float(np.abs(q2t[:, 0] * w).sum())
+    assert abs(lhs - float((q1_ad[:, 0] * dq).sum())) <= DOT_TOL * scale
+
+
+@pytest.mark.parametrize("km", [2, 3, 4, 5, 6, 33])
+def test_state_remap_tangent_matches_the_dual_column(cuda, km):
+    """The state's kord-4 remap tangent (closed forms) against the drop-in's (dual numbers), every column."""
+    import torch
+    n, nq = 12, 2
+    P = S.make_problem(n, km, nq, seed=km)
+    rng = np.random.default_rng(km)
+    host = lambda a: np.array(a.detach().cpu().numpy() if hasattr(a, "detach") else a, dtype=np.float64)
+    q, delp = host(P.q), host(P.dp)
+    q[rng.uniform(size=q.shape) < 0.3] = 0.0
+    dq = rng.standard_normal(q.shape)
+    st = api.CubeState(n, km, nq, precision="fp64", hord=5, kord=4, iv=0)
+    try:
+        st.load_problem(P)
+        st.upload("Q", q)
+        dx = torch.as_tensor(dq, device="cuda")
+        out = torch.zeros_like(dx)
+        st.step_tl(0, dx.data_ptr(), out.data_ptr(), parts=2)
+        got = out.cpu().numpy()
+    finally:
+        st.close()
+    c = slice(3, 3 + n)
+    for t in (0, 4):
+        dp = delp[t][:, c, c].reshape(km, -1)
+        pe1 = np.ascontiguousarray(P.ak[0] + np.concatenate([np.zeros((1, n * n)), np.cumsum(dp, 0)]))
+        pe2 = np.ascontiguousarray(np.asarray(P.ak)[:, None] + np.asarray(P.bk)[:, None] * pe1[-1][None])
+        for iq in range(nq):
+            row = lambda a: np.ascontiguousarray(a[t, iq][:, c, c].reshape(km, 1, -1))
+            ref = np.zeros((km, 1, n * n))
+            api.map1_ppm_tl(km, pe1, row(q), row(dq), None, km, pe2, None, ref, 1, n * n, 1, 1, n * n, 1, 1, 0, 4)
+            assert rel_l2(row(got), ref) <= TL_TOL
+    assert not got[..., :3, :].any() and not got[..., :, n + 3:].any()
