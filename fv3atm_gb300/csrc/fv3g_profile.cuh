@@ -8,7 +8,10 @@
 // limiter is written with selects, so lanes of a warp that take different
 // cases do not diverge.  Sign tests compare the two operands with zero rather
 // than forming their product, which keeps FP32 columns free of underflow in
-// the product (the sign of a difference of two floats is exact).
+// the product (the sign of a difference of two floats is exact).  Tests are joined with
+// & and |, and the column's end interfaces taken by selects: as && and || and early
+// returns they were branches, whose reconvergence was a fifth of the FP32 column kernel's
+// instructions.
 //
 // kord 9.  Interfaces a_u (u = 0..km) come from the C1 tridiagonal system
 // (the kernels solve it).  With D_u = q_u - q_{u-1} the jump across
@@ -53,10 +56,10 @@ template <typename T> __device__ __forceinline__ T sign_of(T a, T b) {
 }
 // x and y of opposite strict signs (x * y < 0 without forming the product)
 template <typename T> __device__ __forceinline__ bool opposite(T x, T y) {
-  return (x > T(0) && y < T(0)) || (x < T(0) && y > T(0));
+  return ((x > T(0)) & (y < T(0))) | ((x < T(0)) & (y > T(0)));
 }
 template <typename T> __device__ __forceinline__ bool same_sign(T x, T y) {
-  return (x > T(0) && y > T(0)) || (x < T(0) && y < T(0));
+  return ((x > T(0)) & (y > T(0))) | ((x < T(0)) & (y < T(0)));
 }
 
 // CW84 eq. 1.10 in perturbation form with selects in place of branches
@@ -76,16 +79,17 @@ template <typename T> __device__ __forceinline__ void cw84_sel(T& bl, T& br) {
 // interface reads layers 0, 1 as qb, qp1, the bottom one km-2, km-1 as qm2, qa)
 template <typename T>
 __device__ __forceinline__ T k9_interface(T a, int u, int km, int iv, T floor_v, T qm2, T qa, T qb, T qp1) {
-  if (u <= 0) return clamp2(a, qb, qp1);
-  if (u >= km) return iv == -2 ? a : clamp2(a, qm2, qa);
+  const bool top = u <= 0, bot = u >= km;
+  const T x0 = top ? qp1 : (bot ? qm2 : qa), x1 = bot ? qa : qb;  // the two means beside the interface
   const T dc = qb - qa;
   const T dl = u > 1 ? qa - qm2 : dc;
   const T dr = u < km - 1 ? qp1 - qb : dc;
-  const T lo = tmin(qa, qb), hi = tmax(qa, qb);
-  const bool mono = same_sign(dl, dr);
-  const bool near_max = !mono && dl > T(0);
-  const T below = tmin(a, hi);
-  return mono ? tmin(tmax(a, lo), hi) : (near_max ? tmax(a, lo) : (iv >= 0 ? tmax(below, floor_v) : below));
+  const T lo = tmin(x0, x1), hi = tmax(x0, x1);
+  const bool mono = top | bot | same_sign(dl, dr);
+  const bool near_max = !mono & (dl > T(0));
+  const T above = tmax(a, lo), below = tmin(a, hi);
+  const T r = mono ? tmin(above, hi) : (near_max ? above : (iv >= 0 ? tmax(below, floor_v) : below));
+  return bot & (iv == -2) ? a : r;
 }
 
 // the same through a layer functor q(k): the end interfaces take their
@@ -171,8 +175,9 @@ template <typename T>
 __device__ __forceinline__ void positivity(T qk, T floor_v, T& bl, T& br) {
   const T s6 = T(-3) * (bl + br), da = br - bl;
   const bool inner = -s6 > tabs(da);
-  const bool low = (qk + bl < floor_v) || (qk + br < floor_v) ||
-                   (inner && T(12) * s6 * (qk - floor_v) + s6 * s6 + T(3) * da * da > T(0));
+  bool low = (qk + bl < floor_v) | (qk + br < floor_v);
+  if (Single<T>::value) low = low | (inner & (T(12) * s6 * (qk - floor_v) + s6 * s6 + T(3) * da * da > T(0)));
+  else low = low || (inner && T(12) * s6 * (qk - floor_v) + s6 * s6 + T(3) * da * da > T(0));
   if (low) {
     T pmin = tmin(qk + bl, qk + br);
     if (inner) pmin = tmin(pmin, qk + pos_div(s6, T(12)) + pos_div(da * da, T(4) * s6));
@@ -191,7 +196,7 @@ template <typename T, int KORD>
 __device__ __forceinline__ void interior_constraint(T qm2, T qm1, T qk, T qp1, T qp2, T dmk, T& bl, T& br) {
   if (KORD == 9) {
     const T Dm = qm1 - qm2, D0 = qk - qm1, D1 = qp1 - qk, D2 = qp2 - qp1;
-    const bool flat = opposite(D0, D1) && (opposite(Dm, D0) || opposite(D1, D2));
+    const bool flat = opposite(D0, D1) & (opposite(Dm, D0) | opposite(D1, D2));
     const bool nonmono = T(3) * tabs(bl + br) > tabs(br - bl);
     const T pr = T(2) * D0, lr = pr - T(1.5) * Dm;
     const T pl = T(-2) * D1, ll = pl + T(1.5) * D2;

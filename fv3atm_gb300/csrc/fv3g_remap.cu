@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "fv3g_ff.cuh"
+#include "fv3g_fp64.cuh"
 #include "fv3g_internal.cuh"
 #include "fv3g_profile.cuh"
 #include "fv3g_remap.cuh"
@@ -231,6 +232,10 @@ __global__ void __launch_bounds__(128) k_remap_scratch(const RemapArgs<T> a) {
 }
 
 // ------------------------------------------------ warp-per-column form ---
+// Bound: issue and latency of the warp's chain (62 % of issue slots, 16 warps an SM).
+// Set-up and passes of 6 x C192 x 127 levels x 9 fields: 4.65 ms before sign tests were
+// joined without branches, the float-float sums of a pass's two fields packed, the layer
+// and mass arrays gathered in 16-byte entries and the results stored by rows; 3.30 ms now.
 // One warp per column; lane l owns interfaces / layers u = l*NPL .. l*NPL+NPL-1,
 // so the column's constants stay in registers for all fields.  The three
 // first-order recurrences of the column are evaluated as warp scans and then
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(128) k_remap_scratch(const RemapArgs<T> a) {
 //   * per field, forward substitution y_u = (rhs_u - y_{u-1}) rd_u and back
 //     substitution a_u = y_u - cp_u a_{u+1}, affine maps composed in the scan.
 // The overlap schedule (source layer and fractional position of every target
-// interface) is a binary search in the warp's copy of pe1.
+// interface) is a short walk in the warp's copy of pe1.
 // Shared arrays indexed by level take one pad element per 32 floats (16
 // doubles), so that lane l reading level 4l+j (the blocked ownership) hits
 // distinct banks.
@@ -254,23 +259,32 @@ __host__ __device__ constexpr int pk(int k) { return k + (k >> (sizeof(T) == 8 ?
 template <typename T>
 __host__ __device__ constexpr int fields_per_pass() { return sizeof(T) == 4 ? 2 : 1; }
 
+// Entry k of the parabola and mass arrays: one pad entry per four, so that lanes four
+// levels apart (16-byte entries) hit distinct banks.
+__host__ __device__ constexpr int px(int k) { return k + (k >> 2); }
+
+// One 16-byte entry per source layer and field, and per source interface, so that a
+// target interface gathers its layer with one load per field.
 template <typename T, int NPL>
-struct ColSmem {
+struct __align__(16) ColSmem {
   static constexpr int FP = fields_per_pass<T>();
-  double pe1[pk<double>(32 * NPL) + 1];
-  T dp[pk<T>(32 * NPL)];
-  T pl[FP][pk<T>(32 * NPL)];  // sub-grid parabola of every source layer: left, right edge and curvature
-  T pr[FP][pk<T>(32 * NPL)];
-  T p6[FP][pk<T>(32 * NPL)];
-  float mh[FP][pk<float>(32 * NPL) + 1];  // FP32 fields: cumulative layer mass at every source interface,
-  float ml[FP][pk<float>(32 * NPL) + 1];  // as an unevaluated sum hi + lo (float-float)
+  float4 par[FP][px(32 * NPL)];  // sub-grid parabola: left, right edge, curvature; the layer's thickness
+  union {
+    float4 mass[px(32 * NPL) + 1];        // cumulative layer mass of the two fields, hi.xy lo.xy (float-float)
+    double pe1[pk<double>(32 * NPL) + 1];  // during the column's set-up
+  };
+  T dp[32 * NPL];
 };
 
 // Fields reach shared memory through a ring of RING slots, filled by
 // cp.async RING-1 fields ahead.  Each slot holds the CTA's 8 columns,
-// [column][padded level].  The CTA's threads copy it together:
+// [column][level].  The CTA's threads copy it together:
 // thread t moves levels t/8 + 32r of column t%8, so 8 consecutive threads read
-// one 32-byte sector (consecutive columns are consecutive i).
+// one 32-byte sector (consecutive columns are consecutive i).  The results take the
+// fields' place in the slots and leave the same way, as do the thicknesses: stored by the
+// lanes that hold them, 4 bytes of 32 different sectors per instruction, they kept the
+// load/store pipe half busy (2 fields of 6 x C192 x 127 levels 0.69 ms, 0.51 ms through
+// the slots).
 template <typename T>
 __host__ __device__ constexpr int ring_slots() { return sizeof(T) == 8 ? 3 : 4; }
 
@@ -279,13 +293,12 @@ __host__ __device__ constexpr int ring_slots() { return sizeof(T) == 8 ? 3 : 4; 
 // 9 % slower at C384 L127 x 20).
 constexpr int RCOL = 8;
 
-// Slot pitch per column: room for the padded levels, and a residue (4 mod 32
-// floats, 2 mod 16 doubles) that spreads the 8 columns of one copy
-// instruction over distinct banks.
+// Slot pitch per column: room for the levels, and a residue (4 mod 32 floats) that
+// spreads the 8 columns of one copy instruction over distinct banks.
 template <typename T, int NPL>
 __host__ __device__ constexpr int ring_pitch() {
-  int p = pk<T>(32 * NPL) + 1;
-  while (sizeof(T) == 8 ? (p % 16 != 2) : (p % 32 != 4)) ++p;
+  int p = 32 * NPL;
+  while (p % 32 != 4) ++p;
   return p;
 }
 
@@ -392,29 +405,30 @@ __device__ __forceinline__ void affine_enter_bwd_m(const T (&m)[5], T (&be)[N], 
   for (int h = 0; h < N; ++h) out[h] = __shfl_down_sync(0xffffffffu, be[h], 1);
 }
 
-template <typename T>
-__device__ __forceinline__ T affine_enter_fwd(T al, T be, int lane) {
+// A lane's NPL levels to and from a column in shared memory, in the widest words NPL allows.
+template <int NPL>
+__device__ __forceinline__ void get_levels(float (&v)[NPL], const float* p) {
+  if constexpr (NPL % 4 == 0) {
+    const float4 x = *(const float4*)p;
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+  } else if constexpr (NPL == 2) {
+    const float2 x = *(const float2*)p;
+    v[0] = x.x, v[1] = x.y;
+  } else {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const T pa = __shfl_up_sync(0xffffffffu, al, o), pb = __shfl_up_sync(0xffffffffu, be, o);
-    if (lane >= o) {
-      be = al * pb + be;
-      al = al * pa;
-    }
+    for (int j = 0; j < NPL; ++j) v[j] = p[j];
   }
-  return __shfl_up_sync(0xffffffffu, be, 1);
 }
-template <typename T>
-__device__ __forceinline__ T affine_enter_bwd(T al, T be, int lane) {
+template <int NPL>
+__device__ __forceinline__ void put_levels(float* p, const float (&v)[NPL]) {
+  if constexpr (NPL % 4 == 0) {
+    *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
+  } else if constexpr (NPL == 2) {
+    *(float2*)p = make_float2(v[0], v[1]);
+  } else {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const T pa = __shfl_down_sync(0xffffffffu, al, o), pb = __shfl_down_sync(0xffffffffu, be, o);
-    if (lane + o < 32) {
-      be = al * pb + be;
-      al = al * pa;
-    }
+    for (int j = 0; j < NPL; ++j) p[j] = v[j];
   }
-  return __shfl_down_sync(0xffffffffu, be, 1);
 }
 
 template <typename T, int KORD, int NPL>  // T: float (FP64 columns: k_remap64)
@@ -428,24 +442,19 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
   const int nc = (int)a.ncol;  // launch_remap checks that it fits in an int
   const int col0 = blockIdx.x * RCOL;
   // the last CTA's surplus warps repeat the last column and store nothing
-  const bool real = col0 + warp < nc;
-  const int col = real ? col0 + warp : nc - 1;
-  auto offsets = [&a](int c, long long& fo_, long long& qo_) {
-    const unsigned ni = (unsigned)a.ni, nj = (unsigned)a.nj;
-    const unsigned rest = (unsigned)c / ni, ci = (unsigned)c - rest * ni;
-    const unsigned ct = rest / nj, cj = rest - ct * nj;
-    fo_ = ct * a.sFt + a.pg.at(a.i1 + ci, a.j1 + cj);
-    qo_ = ct * a.sQt + a.pg.at(a.i1 + ci, a.j1 + cj);
-  };
-  long long fo, qo;
-  offsets(col, fo, qo);
+  const int col = min(col0 + warp, nc - 1);
   const int km = a.km, kn = a.kn;
   const int u0 = lane * NPL;  // first interface / layer of this lane
 
   // cooperative field copy: this thread's column and levels
   const int cc = threadIdx.x % RCOL, kk = threadIdx.x / RCOL;
   long long fo_c, qo_c;
-  offsets(min(col0 + cc, nc - 1), fo_c, qo_c);
+  {
+    const unsigned c = (unsigned)min(col0 + cc, nc - 1), ni = (unsigned)a.ni, nj = (unsigned)a.nj;
+    const unsigned rest = c / ni, ci = c - rest * ni, ct = rest / nj, cj = rest - ct * nj;
+    fo_c = ct * a.sFt + a.pg.at(a.i1 + ci, a.j1 + cj);
+    qo_c = ct * a.sQt + a.pg.at(a.i1 + ci, a.j1 + cj);
+  }
   auto issue = [&](int f) {
     if (f < a.nfield) {
       const T* src = a.q_in + qo_c + f * a.sQq;
@@ -453,13 +462,37 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
 #pragma unroll
       for (int r = 0; r < NPL; ++r) {
         const int k = kk + 32 * r;
-        if (k < km) cp_async_elem(dst + pk<T>(k), src + (long long)k * a.sQk);
+        if (k < km) cp_async_elem(dst + k, src + (long long)k * a.sQk);
       }
     }
     cp_async_commit();
   };
+  // levels 0..nk-1 of this thread's column from slot slot to out; out's column starts at
+  // off.  A slot is refilled by the threads that emptied it, in that order.
+  auto drain = [&](int slot, T* out, long long sk, int nk) {
+    if (col0 + cc >= nc) return;
+    const T* src = ring + (slot * RCOL + cc) * RP;
 #pragma unroll
-  for (int f = 0; f < RING - fields_per_pass<T>(); ++f) issue(f);
+    for (int r = 0; r < NPL; ++r) {
+      const int k = kk + 32 * r;
+      if (k < nk) out[(long long)k * sk] = src[k];
+    }
+  };
+  constexpr int FP = fields_per_pass<T>();
+  static_assert(RING >= 2 * FP && RING - FP >= 2, "two slots are free until the first pass refills them");
+  // the column's thicknesses come through slot RING - 2 and leave through slot RING - 1
+  if (a.pe1 == nullptr) {
+    const T* src = a.dp + fo_c;
+    T* dst = ring + ((RING - 2) * RCOL + cc) * RP;
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) {
+      const int k = kk + 32 * r;
+      if (k < km) cp_async_elem(dst + k, src + (long long)k * a.sFk);
+    }
+  }
+  cp_async_commit();
+#pragma unroll
+  for (int f = 0; f < RING - FP; ++f) issue(f);
 
   // ------------------------------------------------ interface pressures pe1
   if (a.pe1 != nullptr) {
@@ -469,12 +502,20 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
   } else {
     const double ptop = a.ak[0];
     double dl[NPL], tot = 0.0;
+    cp_async_wait<RING - FP>();
+    __syncthreads();
+    T own[NPL];
+    get_levels<NPL>(own, ring + ((RING - 2) * RCOL + warp) * RP + u0);
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
-      dl[j] = (u0 + j < km) ? (double)a.dp[fo + (long long)(u0 + j) * a.sFk] : 0.0;
+      dl[j] = (u0 + j < km) ? (double)own[j] : 0.0;
       tot += dl[j];
     }
-    double excl = affine_enter_fwd<double>(1.0, tot, lane);  // sum over lower lanes
+    for (int o = 1; o < 32; o <<= 1) {  // sum over lower lanes
+      const double below = __shfl_up_sync(0xffffffffu, tot, o);
+      if (lane >= o) tot += below;
+    }
+    const double excl = __shfl_up_sync(0xffffffffu, tot, 1);
     double s = lane == 0 ? ptop : ptop + excl;
     if (lane == 0) S.pe1[pk<double>(0)] = ptop;
 #pragma unroll
@@ -487,37 +528,41 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
   const double ps = S.pe1[pk<double>(km)];
   auto pe2_at = [&](int k) -> double {
     if (a.pe2 != nullptr) return a.pe2[(long long)k * nc + col];
-    return a.ak[k] + a.bk[k] * ps;
+    return __fma_rn(a.bk[k], ps, a.ak[k]);
   };
 #pragma unroll
   for (int j = 0; j < NPL; ++j)
-    if (u0 + j < km) S.dp[pk<T>(u0 + j)] = T(S.pe1[pk<double>(u0 + j + 1)] - S.pe1[pk<double>(u0 + j)]);
+    if (u0 + j < km) S.dp[u0 + j] = T(S.pe1[pk<double>(u0 + j + 1)] - S.pe1[pk<double>(u0 + j)]);
   __syncwarp();
 
   // ----------------------------------------- overlap schedule, target dp
   // Source layer k1 holding target interface p: the number of interior source
   // interfaces at or above p (a short walk from the target's own index).
-  int Ls[NPL + 1];
-  T Xs[NPL + 1], dpk[NPL];
+  // FP64 instructions (16 cycles of an SM each) bound this part, so the walk compares
+  // bit patterns and the layer's thickness comes from S.dp: about 50 of them per warp
+  // instead of 77 (the column set-up of 6 x C192 x 127 levels: 1.07 to 0.75 ms).
+  int Ls[NPL];
+  T Xs[NPL], dpk[NPL];
   double p2v[NPL + 1];
 #pragma unroll
-  for (int j = 0; j <= NPL; ++j) {
+  for (int j = 0; j < NPL; ++j) {
     const int k2 = min(u0 + j, kn);
     const double p = pe2_at(k2);
+    const long long pkey = dkey(p);
     p2v[j] = p;
     int k1 = min(k2, km - 1);
-    while (k1 > 0 && S.pe1[pk<double>(k1)] > p) --k1;
-    while (k1 < km - 1 && S.pe1[pk<double>(k1 + 1)] <= p) ++k1;
-    const double pl = S.pe1[pk<double>(k1)], ph = S.pe1[pk<double>(k1 + 1)];
+    while (k1 > 0 && dkey(S.pe1[pk<double>(k1)]) > pkey) --k1;
+    while (k1 < km - 1 && dkey(S.pe1[pk<double>(k1 + 1)]) <= pkey) ++k1;
     Ls[j] = k1;
-    Xs[j] = Single<T>::value ? T(float(p - pl) / float(ph - pl)) : T((p - pl) / (ph - pl));
+    Xs[j] = T(float(p - S.pe1[pk<double>(k1)]) / (float)S.dp[k1]);
   }
+  p2v[NPL] = __shfl_down_sync(0xffffffffu, p2v[0], 1);  // 32 NPL > kn: lane 31's is never used
 #pragma unroll
   for (int j = 0; j < NPL; ++j) {
     const int t = u0 + j;
     dpk[j] = (t < kn) ? (a.dp2 ? T(a.dp2[(long long)t * nc + col]) : T(p2v[j + 1] - p2v[j])) : T(1);
-    if (real && t < kn && a.dp_out != nullptr) a.dp_out[fo + (long long)t * a.sFk] = dpk[j];
   }
+  if (a.dp_out != nullptr) put_levels<NPL>(ring + ((RING - 1) * RCOL + warp) * RP + u0, dpk);
 
   // ------------------------------------------- LU of the interface system
   // Row u of the system: rhs_u = wa q_a + wb q_b + wc qs with layers a, b =
@@ -529,13 +574,13 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
 #pragma unroll
   for (int j = 0; j < NPL; ++j) wa[j] = wb[j] = wc[j] = mco[j] = rdv[j] = cpb[j] = T(0);
   if (KORD == 9 && km > 1) {
-    const T g = S.dp[pk<T>(1)] / S.dp[pk<T>(0)];
+    const T g = S.dp[1] / S.dp[0];
     T dd[NPL];
     Mat2<T> m{T(1), T(0), T(0), T(1)};
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
       const int u = u0 + j;
-      dd[j] = (u >= 1 && u < km) ? S.dp[pk<T>(u - 1)] / S.dp[pk<T>(u)] : T(0);
+      dd[j] = (u >= 1 && u < km) ? S.dp[u - 1] / S.dp[u] : T(0);
       if (u >= 1 && u < km) m = mat_after(Mat2<T>{T(0), dd[j], T(-1), T(2) * (T(1) + dd[j])}, m);
     }
 #pragma unroll
@@ -546,7 +591,7 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
     const Mat2<T> e = shfl_up_mat(m, 1);
     const T cp0 = (g + T(1)) / g;
     T cprev = (e.a * cp0 + e.b) / (e.c * cp0 + e.d);  // cp of interface u0-1 (lanes >= 1)
-    const T gb = S.dp[pk<T>(km - 2)] / S.dp[pk<T>(km - 1)];
+    const T gb = S.dp[km - 2] / S.dp[km - 1];
     const T lo_b = a.iv == -2 ? T(0) : gb + T(1);
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
@@ -578,9 +623,12 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
 
   const T floor_v = (a.iv == 1) ? T(a.q_min) : T(0);
   const T qsv = a.qs ? T(a.qs[col]) : T(0);
-  T rdpk[NPL];
+  T rdpk[NPL], dpl[NPL];  // reciprocal target thickness; source thickness (0 past km)
 #pragma unroll
-  for (int j = 0; j < NPL; ++j) rdpk[j] = T(1) / dpk[j];
+  for (int j = 0; j < NPL; ++j) {
+    rdpk[j] = T(1) / dpk[j];
+    dpl[j] = u0 + j < km ? S.dp[u0 + j] : T(0);
+  }
   // the substitution scans' multipliers (column constants): forward a_j = -mco_j rd_j, backward -cp_j
   T ajv[NPL], mf[5], mb[5];
   {
@@ -598,32 +646,49 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
   // kord 4: thicknesses of layers u0-2 .. u0+NPL+1 (clamped into the column)
   T hw[NPL + 4];
 #pragma unroll
-  for (int i = 0; i < NPL + 4; ++i) hw[i] = KORD == 9 ? T(1) : S.dp[pk<T>(min(max(u0 - 2 + i, 0), km - 1))];
-  constexpr int FP = fields_per_pass<T>();
+  for (int i = 0; i < NPL + 4; ++i) hw[i] = KORD == 9 ? T(1) : S.dp[min(max(u0 - 2 + i, 0), km - 1)];
   for (int f0 = 0; f0 < a.nfield; f0 += FP) {
-    __syncthreads();  // every warp is done with the previous pass, whose slots are refilled now
+    __syncthreads();  // every warp is done with the previous pass: its results leave, its slots are refilled
+    if (f0 > 0) {
+#pragma unroll
+      for (int h = 0; h < FP; ++h) drain((f0 - FP + h) % RING, a.q_out + qo_c + (f0 - FP + h) * a.sQqo, a.sQk, kn);
+    } else if (a.dp_out != nullptr) {
+      drain(RING - 1, a.dp_out + fo_c, a.sFk, kn);
+    }
 #pragma unroll
     for (int h = 0; h < FP; ++h) issue(f0 + RING - FP + h);
     cp_async_wait<RING - FP>();
     __syncthreads();  // the pass's fields are in their slots
-    // a pass past the last field repeats it and stores nothing
-    const T* Q[FP];
-    T* q2[FP];
-    bool store[FP];
+    // a pass past the last field repeats it and stores nothing; the results take the place of
+    // the fields in their slots
+    T* Q[FP];
 #pragma unroll
     for (int h = 0; h < FP; ++h) {
       const int f = min(f0 + h, a.nfield - 1);
       Q[h] = ring + ((f % RING) * RCOL + warp) * RP;
-      q2[h] = a.q_out + qo + f * a.sQqo;
-      store[h] = real && f0 + h < a.nfield;
     }
     // w[h][i]: mean of layer u0 - 2 + i (clamped into the column), the lane's
     // layers and two on either side; qv: the lane's own layers (0 past km)
     T qv[FP][NPL], st[FP][NPL], w[FP][NPL + 4];
 #pragma unroll
     for (int h = 0; h < FP; ++h) {
+      if constexpr (NPL % 2 == 0) {  // 16- or 8-byte loads, then the clamps
+        const float2 lo = *(const float2*)(Q[h] + max(u0 - 2, 0)), hi = *(const float2*)(Q[h] + min(u0 + NPL, RP - 2));
+        const T last = Q[h][km - 1];
+        T own[NPL];
+        get_levels<NPL>(own, Q[h] + u0);
 #pragma unroll
-      for (int i = 0; i < NPL + 4; ++i) w[h][i] = Q[h][pk<T>(min(max(u0 - 2 + i, 0), km - 1))];
+        for (int j = 0; j < NPL; ++j) w[h][j + 2] = own[j];
+        w[h][0] = lane == 0 ? w[h][2] : lo.x;
+        w[h][1] = lane == 0 ? w[h][2] : lo.y;
+        w[h][NPL + 2] = hi.x;
+        w[h][NPL + 3] = hi.y;
+#pragma unroll
+        for (int i = 0; i < NPL + 4; ++i) w[h][i] = u0 - 2 + i < km ? w[h][i] : last;
+      } else {
+#pragma unroll
+        for (int i = 0; i < NPL + 4; ++i) w[h][i] = Q[h][min(max(u0 - 2 + i, 0), km - 1)];
+      }
 #pragma unroll
       for (int j = 0; j < NPL; ++j) qv[h][j] = (u0 + j < km) ? w[h][j + 2] : T(0);
     }
@@ -701,8 +766,8 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
           dmw[i] = (k >= 1 && k <= km - 2) ? m : T(0);
         }
         const T* Qh = Q[h];
-        auto qf = [Qh, km](int k) -> T { return Qh[pk<T>(min(max(k, 0), km - 1))]; };
-        auto hf = [&S, km](int k) -> T { return S.dp[pk<T>(min(max(k, 0), km - 1))]; };
+        auto qf = [Qh, km](int k) -> T { return Qh[min(max(k, 0), km - 1)]; };
+        auto hf = [&S, km](int k) -> T { return S.dp[min(max(k, 0), km - 1)]; };
         T ai[NPL + 1];
 #pragma unroll
         for (int j = 0; j <= NPL; ++j) {
@@ -739,11 +804,7 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
         bl = end ? ble : bl;
         br = end ? bre : br;
         if (a.iv >= 0) positivity(qk, floor_v, bl, br);
-        if (u < km) {
-          S.pl[h][pk<T>(u)] = qk + bl;
-          S.pr[h][pk<T>(u)] = qk + br;
-          S.p6[h][pk<T>(u)] = T(-3) * (bl + br);
-        }
+        S.par[h][px(u)] = make_float4(qk + bl, qk + br, T(-3) * (bl + br), dpl[j]);
       }
     }
     {
@@ -751,82 +812,75 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
       // interface (layer masses q*dp are exact as float-float products), so a
       // target layer's mass is a difference of two cumulative values and the
       // column mass telescopes; only the final division rounds per value.
-      FF m[FP][NPL], ex[FP];
+      static_assert(FP == 2, "two fields in lockstep");
+      FFP m[NPL], ex{bc(0.f), bc(0.f)};
 #pragma unroll
-      for (int h = 0; h < FP; ++h) {
-        ex[h] = FF{0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < NPL; ++j) {
-          m[h][j] = (u0 + j < km) ? ff_prod((float)qv[h][j], (float)S.dp[pk<T>(u0 + j)]) : FF{0.f, 0.f};
-          ex[h] = ff_add(ex[h], m[h][j]);
-        }
+      for (int j = 0; j < NPL; ++j) {
+        m[j] = ffp_prod(F2{qv[0][j], qv[1][j]}, dpl[j]);
+        ex = ffp_add(ex, m[j]);
       }
       // inclusive scan of the lane totals, then shifted by one lane
+      auto up = [](F2 v, int o) {
+        return F2{__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o)};
+      };
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        FF p[FP];
-#pragma unroll
-        for (int h = 0; h < FP; ++h)
-          p[h] = FF{__shfl_up_sync(0xffffffffu, ex[h].hi, o), __shfl_up_sync(0xffffffffu, ex[h].lo, o)};
-#pragma unroll
-        for (int h = 0; h < FP; ++h)
-          if (lane >= o) ex[h] = ff_add(p[h], ex[h]);
+        const FFP p{up(ex.hi, o), up(ex.lo, o)};
+        const bool in = lane >= o;  // adding zero leaves a sum as it is
+        ex = ffp_add(FFP{F2{in ? p.hi.x : 0.f, in ? p.hi.y : 0.f}, F2{in ? p.lo.x : 0.f, in ? p.lo.y : 0.f}}, ex);
       }
+      FFP run{up(ex.hi, 1), up(ex.lo, 1)};
+      if (lane == 0) run = FFP{bc(0.f), bc(0.f)};
 #pragma unroll
-      for (int h = 0; h < FP; ++h) {
-        FF run{__shfl_up_sync(0xffffffffu, ex[h].hi, 1), __shfl_up_sync(0xffffffffu, ex[h].lo, 1)};
-        if (lane == 0) run = FF{0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < NPL; ++j) {
-          if (u0 + j <= km) {
-            S.mh[h][pk<float>(u0 + j)] = run.hi;
-            S.ml[h][pk<float>(u0 + j)] = run.lo;
-          }
-          run = ff_add(run, m[h][j]);
-        }
+      for (int j = 0; j < NPL; ++j) {
+        S.mass[px(u0 + j)] = make_float4(run.hi.x, run.hi.y, run.lo.x, run.lo.y);
+        if (j + 1 < NPL) run = ffp_add(run, m[j]);
       }
     }
     __syncwarp();
     // ------------------------------------------------------- integration
+    {
+      // cumulative mass at this lane's target interfaces (a layer wholly above one: the mass
+      // at the next interface, nothing added); the last one is the next lane's first (32 NPL >
+      // kn, so lane 31's last is never used)
+      FFP cm[NPL + 1];
 #pragma unroll
-    for (int h = 0; h < FP; ++h) {
-      {
-        // cumulative mass at this lane's target interfaces; the last one is the
-        // next lane's first (32 NPL > kn, so lane 31's last is never used)
-        FF cm[NPL + 1];
-#pragma unroll
-        for (int j = 0; j < NPL; ++j) {
-          const int L = Ls[j];
-          const float X = (float)Xs[j];
-          const int il = pk<float>(L), iu = pk<float>(L + 1);
-          FF c{S.mh[h][il], S.ml[h][il]};
-          if (X >= 1.f) {
-            c = FF{S.mh[h][iu], S.ml[h][iu]};
-          } else if (X > 0.f) {
-            const int it = pk<T>(L);
-            const float part =
-                (float)S.dp[it] * X * (float)pmean(S.pl[h][it], S.pr[h][it], S.p6[h][it], T(0), T(X));
-            c = ff_add(c, FF{part, 0.f});
-          }
-          cm[j] = c;
-        }
-        cm[NPL] = FF{__shfl_down_sync(0xffffffffu, cm[0].hi, 1), __shfl_down_sync(0xffffffffu, cm[0].lo, 1)};
-#pragma unroll
-        for (int j = 0; j < NPL; ++j) {
-          const int t = u0 + j;
-          const FF mass = ff_add(cm[j + 1], ff_neg(cm[j]));
-          // the quotient mass / dp, not mass times the rounded reciprocal (that rounding is shared by every
-          // tracer of the layer and biased the global mass, +5e-10 per step at C384 L127 x20): the
-          // reciprocal's product corrected by one Newton step on the exact residual (fma), which gives the
-          // rounded quotient but for rare ties, unbiased
-          const float mm = mass.hi + mass.lo, d = (float)dpk[j], r = (float)rdpk[j];
-          const float q0 = mm * r;
-          const float qq = fmaf(fmaf(-q0, d, mm), r, q0);
-          if (store[h] && t < kn) q2[h][(long long)t * a.sQk] = T(qq);
-        }
+      for (int j = 0; j < NPL; ++j) {
+        const int L = Ls[j];
+        const float X = (float)Xs[j];
+        const bool full = X >= 1.f;
+        const bool cut = (X > 0.f) & !full;
+        const float4 p0 = S.par[0][px(L)], p1 = S.par[1][px(L)], mc = S.mass[px(L + (full ? 1 : 0))];
+        const float dX = p0.w * X;
+        F2 part{dX * pmean(p0.x, p0.y, p0.z, 0.f, X), dX * pmean(p1.x, p1.y, p1.z, 0.f, X)};
+        part = F2{cut ? part.x : 0.f, cut ? part.y : 0.f};
+        cm[j] = ffp_addf(FFP{F2{mc.x, mc.y}, F2{mc.z, mc.w}}, part);
       }
+      auto down = [](F2 v) {
+        return F2{__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1)};
+      };
+      cm[NPL] = FFP{down(cm[0].hi), down(cm[0].lo)};
+#pragma unroll
+      for (int j = 0; j < NPL; ++j) {
+        const FFP mass = ffp_sub(cm[j + 1], cm[j]);
+        // the quotient mass / dp, not mass times the rounded reciprocal (that rounding is shared by every
+        // tracer of the layer and biased the global mass, +5e-10 per step at C384 L127 x20): the
+        // reciprocal's product corrected by one Newton step on the exact residual (fma), which gives the
+        // rounded quotient but for rare ties, unbiased
+        const F2 mm = add2(mass.hi, mass.lo), r = bc((float)rdpk[j]), q0 = mul2(mm, r);
+        const F2 qq = fma2(fma2(q0, bc(-(float)dpk[j]), mm), r, q0);
+        qv[0][j] = qq.x;
+        qv[1][j] = qq.y;
+      }
+      put_levels<NPL>(Q[0] + u0, qv[0]);
+      if (f0 + 1 < a.nfield) put_levels<NPL>(Q[1] + u0, qv[1]);
     }
   }
+  __syncthreads();
+  const int fl = (a.nfield - 1) / FP * FP;
+#pragma unroll
+  for (int h = 0; h < FP; ++h)
+    if (fl + h < a.nfield) drain((fl + h) % RING, a.q_out + qo_c + (fl + h) * a.sQqo, a.sQk, kn);
 }
 
 template <typename T, int KORD, int NPL>
@@ -841,7 +895,8 @@ int prepare_remap_kernels() {
   static std::once_flag once;
   static cudaError_t err = cudaSuccess;
   std::call_once(once, [] {
-    cudaError_t es[] = {set_remap_attr<float, 9, 4>(), set_remap_attr<float, 9, 5>(), set_remap_attr<float, 4, 4>(),
+    cudaError_t es[] = {set_remap_attr<float, 9, 2>(), set_remap_attr<float, 9, 3>(), set_remap_attr<float, 4, 2>(),
+                        set_remap_attr<float, 4, 3>(), set_remap_attr<float, 9, 4>(), set_remap_attr<float, 9, 5>(), set_remap_attr<float, 4, 4>(),
                         set_remap_attr<float, 4, 5>(), prepare_remap64()};
     for (cudaError_t e : es)
       if (e != cudaSuccess && err == cudaSuccess) err = e;
@@ -857,9 +912,14 @@ static cudaError_t launch_warp_npl(const RemapArgs<T>& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Levels a lane holds: the fewest that hold the column, so that no lanes idle (6 x C96, kord 9:
+// 33 levels x 3 fields 0.43 ms with four, 0.26 ms with two; 64 x 4 0.45 and, with three, 0.35 ms).
 template <typename T, int KORD>
 static cudaError_t launch_warp_form(const RemapArgs<T>& a, cudaStream_t s) {
-  if (std::max(a.km, a.kn) < 32 * 4) return launch_warp_npl<T, KORD, 4>(a, s);
+  const int k = std::max(a.km, a.kn);
+  if (k < 32 * 2) return launch_warp_npl<T, KORD, 2>(a, s);
+  if (k < 32 * 3) return launch_warp_npl<T, KORD, 3>(a, s);
+  if (k < 32 * 4) return launch_warp_npl<T, KORD, 4>(a, s);
   return launch_warp_npl<T, KORD, 5>(a, s);
 }
 
