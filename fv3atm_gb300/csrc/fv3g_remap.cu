@@ -960,10 +960,54 @@ int launch_remap(const RemapArgs<T>& a, int kord, cudaStream_t s) {
 // sum of dp (the mean of the two columns beside a face), pe2 = ak + bk ps with
 // the same ps; with log_p both in ln p.  [k][col] layout, col = (t nj + cj) ni
 // + ci over the kind's columns ci < ni, cj < nj.
-template <typename T>
-__global__ void k_field_pressures(const T* dp, long long sFt, long long sFk, PlaneGeom pg, int nt, int km, int ni,
-                                  int nj, int kind, int log_p, const double* ak, const double* bk, double* pe1,
-                                  double* pe2) {
+//
+// Bound: FP64 instructions (16 cycles of an SM each).  CUDA's log takes about 33 of them,
+// ln_tab 11; beside a face the two columns' thicknesses are summed before the running
+// sum, and halved by the exponent.  6 x C192 x 127 levels: cells in ln p 3.73 to 1.33 ms,
+// faces 0.49 to 0.30 ms.
+constexpr int LN_N = 1024;  // table entries: one per 2^-10 of the significand
+
+// ln p by table (Tang 1990): the significand m in [0.75, 1.5) times the tabulated
+// reciprocal r of its bin leaves 1 + e with |e| < 2^-10, and ln p = k ln 2 - ln r + ln(1 +
+// e), the last as its Taylor polynomial of degree 6 (error 2^-63 relative).  k ln 2 is split so
+// that its leading part is exact; the two bins beside 1 have r = 1, which keeps the
+// result's relative error there.  Error below 1 ulp, 0.53 above 1 kPa.  Zero, negative, subnormal, infinite and NaN p
+// go to log.
+__device__ __forceinline__ double ln_tab(double p, const double2* tab) {
+  const int hi = __double2hiint(p);
+  if ((unsigned)(hi - 0x00100000) >= 0x7fe00000u) return log(p);
+  const int up = (hi >> 19) & 1;  // significand from 1.5 on: halved
+  const float kf = (float)((hi >> 20) - 1023 + up);
+  const unsigned kb = __float_as_uint(kf);
+  const double k = __hiloint2double(kf == 0.f ? 0 : (int)(((kb & 0x7fffffffu) >> 3) + (896u << 20) | (kb & 0x80000000u)),
+                                    (int)(kb << 29));
+  const double m = __hiloint2double((hi & 0x000fffff) | (up ? 0x3fe00000 : 0x3ff00000), __double2loint(p));
+  const double2 t = tab[(hi >> 10) & (LN_N - 1)];
+  const double e = fma(m, t.x, -1.0);
+  double c = fma(e, -1.0 / 6.0, 1.0 / 5.0);
+  c = fma(e, c, -1.0 / 4.0);
+  c = fma(e, c, 1.0 / 3.0);
+  c = fma(e, c, -0.5);
+  const double l = fma(e * e, c, e);
+  constexpr double LN2_HI = 0x1.62e42fefa38p-1, LN2_LO = 0x1.ef35793c7673p-45;  // ln 2: 42 bits and the rest
+  return fma(k, LN2_HI, t.y + fma(k, LN2_LO, l));
+}
+__device__ __forceinline__ void ln_table(double2* tab) {
+  for (int i = threadIdx.x; i < LN_N; i += blockDim.x) {
+    const float c = 1.f + (i + 0.5f) / LN_N;  // the bin's middle; halved from 1.5 on
+    const double r = i == 0 || i == LN_N - 1 ? 1.0 : (double)(1.f / (i >= LN_N / 2 ? 0.5f * c : c));
+    tab[i] = make_double2(r, -log(r));
+  }
+  __syncthreads();
+}
+
+template <typename T, bool LOGP, bool FACE>
+__global__ void __launch_bounds__(256) k_field_pressures(const T* dp, long long sFt, long long sFk, PlaneGeom pg, int nt,
+                                                         int km, int ni, int nj, int kind, const double* ak,
+                                                         const double* bk, double* pe1, double* pe2) {
+  __shared__ double2 tab[LOGP ? LN_N : 1];
+  if (LOGP) ln_table(tab);
+  auto out = [&](double p) -> double { return LOGP ? ln_tab(p, tab) : p; };
   const long long nc = (long long)nt * ni * nj;
   const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= nc) return;
@@ -972,20 +1016,18 @@ __global__ void k_field_pressures(const T* dp, long long sFt, long long sFk, Pla
   const int cj = (int)(rest % nj), t = (int)(rest / nj);
   const int i = 1 + ci, j = 1 + cj;
   const T* da = dp + t * sFt + pg.at(i, j);
-  const T* db = dp + t * sFt + (kind == 1 ? pg.at(i, j - 1) : kind == 2 ? pg.at(i - 1, j) : pg.at(i, j));
-  double pa = ak[0], pb = ak[0];
-  pe1[col] = log_p ? log(pa) : pa;
+  const T* db = dp + t * sFt + (kind == 1 ? pg.at(i, j - 1) : pg.at(i - 1, j));
+  double s = FACE ? 2.0 * ak[0] : ak[0];  // beside a face: the sum of the two columns' pressures
+  auto p_of = [](double v) { return FACE ? scale2<-1>(v) : v; };
+  pe1[col] = out(p_of(s));
+#pragma unroll 4
   for (int k = 0; k < km; ++k) {
-    pa += (double)da[(long long)k * sFk];
-    pb += (double)db[(long long)k * sFk];
-    const double p = kind == 0 ? pa : 0.5 * (pa + pb);
-    pe1[(long long)(k + 1) * nc + col] = log_p ? log(p) : p;
+    s += FACE ? (double)da[(long long)k * sFk] + (double)db[(long long)k * sFk] : (double)da[(long long)k * sFk];
+    pe1[(long long)(k + 1) * nc + col] = out(p_of(s));
   }
-  const double ps = kind == 0 ? pa : 0.5 * (pa + pb);
-  for (int k = 0; k <= km; ++k) {
-    const double p = ak[k] + bk[k] * ps;
-    pe2[(long long)k * nc + col] = log_p ? log(p) : p;
-  }
+  const double ps = p_of(s);
+#pragma unroll 4
+  for (int k = 0; k <= km; ++k) pe2[(long long)k * nc + col] = out(fma(bk[k], ps, ak[k]));
 }
 
 template <typename T>
@@ -993,8 +1035,9 @@ int launch_field_pressures(const T* dp, long long sFt, long long sFk, PlaneGeom 
                            int kind, int log_p, const double* ak, const double* bk, double* pe1, double* pe2,
                            cudaStream_t s) {
   const long long nc = (long long)nt * ni * nj;
-  k_field_pressures<T><<<(unsigned)((nc + 127) / 128), 128, 0, s>>>(dp, sFt, sFk, pg, nt, km, ni, nj, kind, log_p, ak,
-                                                                   bk, pe1, pe2);
+  auto kern = kind == 0 ? (log_p ? k_field_pressures<T, true, false> : k_field_pressures<T, false, false>)
+                        : (log_p ? k_field_pressures<T, true, true> : k_field_pressures<T, false, true>);
+  kern<<<(unsigned)((nc + 255) / 256), 256, 0, s>>>(dp, sFt, sFk, pg, nt, km, ni, nj, kind, ak, bk, pe1, pe2);
   FV3G_CUDA(cudaGetLastError());
   return 0;
 }
