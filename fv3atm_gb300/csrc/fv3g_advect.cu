@@ -229,7 +229,7 @@ static void edge_free_range(int is, int ie, int np, int nested, int nb, int& lo,
 }
 
 BlockMap block_map(int is, int ie, int js, int je, int npx, int npy, int nested) {
-  BlockMap m;
+  BlockMap m{};
   m.nbx = (ie - is + TW) / TW;
   m.nby = (je - js + TW) / TW;
   edge_free_range(is, ie, npx, nested, m.nbx, m.bx0, m.nbxi);

@@ -128,6 +128,7 @@ __device__ __forceinline__ void raise_error(int* err, int code) {
 // contains no cube-face edge.
 struct BlockMap {
   int nbx, nby, bx0, nbxi, by0, nbyi;
+  int shift;  // the last column and row of tiles start TW cells before the edge and own only what no other tile does
 };
 
 // Window face (1..31) of the low / high cube-face edge seen by a CTA tile

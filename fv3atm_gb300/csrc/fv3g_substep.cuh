@@ -130,9 +130,8 @@ __device__ __forceinline__ T generic_br(int c, EX&& x) {
   return T(7.0 / 12.0) * (x(c) + x(c + 1)) - T(1.0 / 12.0) * (x(c - 1) + x(c + 2)) - x(c);
 }
 
-template <typename T, int HORD, int OS = 32, class EX, class ED>
-__device__ __noinline__ void edge_devs(int e, bool east, EX x, ED ed, T* o) {
-  if (e == NO_EDGE) return;
+template <typename T, int HORD, int OS, class EX, class ED>
+__device__ __forceinline__ void edge_devs_body(int e, bool east, EX x, ED ed, T* o) {
   bool need[4];
   for (int c = 0; c < 4; ++c) need[c] = (e - 2 + c >= 2 && e - 2 + c <= 29);
   T b[4] = {T(0), T(0), T(0), T(0)}, r[4] = {T(0), T(0), T(0), T(0)};
@@ -187,6 +186,24 @@ __device__ __noinline__ void edge_devs(int e, bool east, EX x, ED ed, T* o) {
   }
   for (int c = 0; c < 4; ++c) { o[c * OS] = b[c]; o[(4 + c) * OS] = r[c]; }
 }
+template <typename T, int HORD, int OS = 32, class EX, class ED>
+__device__ __noinline__ void edge_devs(int e, bool east, EX x, ED ed, T* o) {
+  if (e != NO_EDGE) edge_devs_body<T, HORD, OS>(e, east, x, ed, o);
+}
+// the edges of fixed_edges launches: faces 3 and 29
+constexpr int E_LO = 3, E_HI = 3 + TW;
+// One function each for the lines of all three stages (a line of cells x, SX apart; the edge metrics ed of the four
+// cells): the ring kernel's code is larger than the instruction cache holds comfortably.
+template <typename T, int HORD>
+__device__ __noinline__ void edge_devs_lo(const T* x, int sx, const T* ed, T* o) {
+  edge_devs_body<T, HORD, 32>(E_LO, false, [=](int m) { return x[m * sx]; },
+                              [=](int m) { return ed[(m - E_LO + 2) * WIN]; }, o);
+}
+template <typename T, int HORD>
+__device__ __noinline__ void edge_devs_hi(const T* x, int sx, const T* ed, T* o) {
+  edge_devs_body<T, HORD, 32>(E_HI, true, [=](int m) { return x[m * sx]; },
+                              [=](int m) { return ed[(m - E_HI + 2) * WIN]; }, o);
+}
 
 // A line of 32 window cells x[0..31] marched with a rolling register window;
 // face f separates cells f-1 and f, and faces 3..29 are the CTA tile's.
@@ -206,12 +223,29 @@ __device__ __forceinline__ T dm_clamp(T xm, T x0, T xp) {
   return copysign_t(tmin3(tabs(xt), tmax3(xm, x0, xp) - x0, x0 - tmin3(xm, x0, xp)), xt);
 }
 
+// What a kernel knows of the cube-face edges in its windows: none there; at any face; at face
+// 3 or 29 only, known by tile (fixed_edges), so that the steps that take edge deviations
+// are known when the march is compiled.
+enum { NO_EDGES = 0, ANY_EDGES = 1, FIXED_EDGES = 2 };
+
 // Steps of a line whose cell m-2 lies next to a cube-face edge: bit m of
 // mask, for the two edges at window faces eA and eB (warp-uniform).
 struct EdgeSel {
   unsigned mask;
   int eA, eB;
   int sb;  // first slot of edge B: 8 when a window can hold both edges, else 0
+  // the slot of cell m-2's deviations, -1 if it is not beside an edge
+  template <int EDGES>
+  __device__ __forceinline__ int slot(int m) const {
+    if (EDGES == FIXED_EDGES) {
+      if (m >= E_LO && m < E_LO + 4) return eA != NO_EDGE ? m - E_LO : -1;
+      if (m >= E_HI) return eB != NO_EDGE ? m - E_HI : -1;
+      return -1;
+    }
+    if (EDGES == NO_EDGES || !((mask >> m) & 1u)) return -1;
+    const int dA = m - eA;  // cell e-2+d of an edge
+    return (unsigned)dA < 4u ? dA : sb + (m - eB);
+  }
 };
 __device__ __forceinline__ EdgeSel edge_sel(int eA, int eB, int sb) {
   auto bits = [](int e) { return (e >= 0 && e < 32) ? (0xFu << e) : 0u; };
@@ -231,7 +265,7 @@ struct Line {
   }
 
   // ed: this lane's edge deviations (lane-strided slots: edge A bl0..3 br0..3, then edge B from slot sb)
-  template <bool EDGES>
+  template <int EDGES>
   __device__ __forceinline__ T step(int m, T x, T c, const T* ed, const EdgeSel& es) {
     T alc, bl, br;
     if (HORD == 8) {
@@ -247,9 +281,7 @@ struct Line {
       bl = alb - xb;
       br = alc - xb;
     }
-    if (EDGES && ((es.mask >> m) & 1u)) {  // cell m-2 is cell e-2+d of an edge
-      const int dA = m - es.eA;
-      const int slot = (unsigned)dA < 4u ? dA : es.sb + (m - es.eB);
+    if (const int slot = es.slot<EDGES>(m); EDGES && slot >= 0) {
       bl = ed[slot * 32];
       br = ed[(slot + 4) * 32];
     }
@@ -295,11 +327,11 @@ struct PairLine {
 
   // ed: the pair's edge-deviation slots (lane-strided pairs); or, for two
   // lines with separate slots, edx for the first value and edy for the second
-  template <bool EDGES>
+  template <int EDGES>
   __device__ __forceinline__ F2 step(int m, F2 x, float c, const F2* ed, const EdgeSel& es) {
     return step2<EDGES, true>(m, x, c, ed, nullptr, nullptr, es);
   }
-  template <bool EDGES, bool PAIRED_SLOTS>
+  template <int EDGES, bool PAIRED_SLOTS>
   __device__ __forceinline__ F2 step2(int m, F2 x, float c, const F2* ed, const float* edx, const float* edy,
                                       const EdgeSel& es) {
     // monotonized central slope of cell m-1 (half increments), |dm| and sign
@@ -315,9 +347,7 @@ struct PairLine {
     dmb = dmc;
     mb = mag;
     sb = sg;
-    if (EDGES && ((es.mask >> m) & 1u)) {  // cell m-2 is cell e-2+d of an edge
-      const int dA = m - es.eA;
-      const int slot = (unsigned)dA < 4u ? dA : es.sb + (m - es.eB);
+    if (const int slot = es.slot<EDGES>(m); EDGES && slot >= 0) {
       if (PAIRED_SLOTS) {
         bl = ed[slot * 32];
         br = ed[(slot + 4) * 32];
@@ -353,10 +383,10 @@ __device__ __forceinline__ void stage_ld(T* dst, const T* base, const PlaneGeom&
 
 // ------------------------------------------------------------ the kernel ---
 // One tracer of one CTA tile through the three stages (see file header).
-template <typename T, int HORD, bool FLUXES, bool EDGES>
+template <typename T, int HORD, bool FLUXES, int EDGES>
 __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>& L, SmemWarp<T>& S, int t, int k,
                                                T* eds, int iq, int i0, int j0, int ni, int nj, int lane, int exA,
-                                               int exB, int eyA, int eyB, bool corner_block,
+                                               int exB, int eyA, int eyB, bool corner_block, int c0, int r0,
                                                long long efo, long long efe, int nslot) {
   const PlaneGeom& pg = a.pg;
   const int n = a.npx - 1;
@@ -378,6 +408,13 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
     const int ic = min(max(i0 - 3 + lane, pg.isd), pg.isd + pg.pitch - 1);
     const T* src = base + t * a.sQt + iq * a.sQq + k * a.sQk + (ic - pg.isd);
     const int jhi = pg.jsd + pg.rows - 1;
+    if (j0 - 3 >= pg.jsd && j0 + WIN - 4 <= jhi) {
+      const T* row = src + (long long)(j0 - 3 - pg.jsd) * pg.pitch;
+#pragma unroll 8
+      for (int r = 0; r < WIN; ++r, row += pg.pitch) copy_async(&S.q[r][lane], row);
+      stage_wait();
+      return;
+    }
     // every row in flight (asynchronous copies wait for nothing in the loop and hold no registers), then
     // one wait for them all: the corner cells written next must land after the copies
 #pragma unroll 8
@@ -405,8 +442,13 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
       auto ex = [qcol](int m) { return qcol[m * PQ]; };
       auto edA = [&L, w, eyA](int m) { return L.edy[0][m - eyA + 2][w]; };
       auto edB = [&L, w, eyB](int m) { return L.edy[1][m - eyB + 2][w]; };
-      edge_devs<T, HORD>(eyA, false, ex, edA, ed0);
-      edge_devs<T, HORD>(eyB, true, ex, edB, ed0 + sb * 32);
+      if constexpr (EDGES == FIXED_EDGES) {
+        if (eyA != NO_EDGE) edge_devs_lo<T, HORD>(qcol, PQ, &L.edy[0][0][w], ed0);
+        if (eyB != NO_EDGE) edge_devs_hi<T, HORD>(qcol, PQ, &L.edy[1][0][w], ed0);
+      } else {
+        edge_devs<T, HORD>(eyA, false, ex, edA, ed0);
+        edge_devs<T, HORD>(eyB, true, ex, edB, ed0 + sb * 32);
+      }
     }
     Line<T, HORD> ln;
     ln.init(T(a.lim_fac));
@@ -447,14 +489,25 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
       auto exo = [qirow](int m) { return qirow[m]; };
       auto edA = [&L, r, exA](int m) { return L.edx[0][m - exA + 2][r]; };
       auto edB = [&L, r, exB](int m) { return L.edx[1][m - exB + 2][r]; };
-      edge_devs<T, HORD>(exA, false, exi, edA, ed0);
-      edge_devs<T, HORD>(exB, true, exi, edB, ed0 + sb * 32);
-      if (outer) {
-        edge_devs<T, HORD>(exA, false, exo, edA, ed1);
-        edge_devs<T, HORD>(exB, true, exo, edB, ed1 + sb * 32);
+      if constexpr (EDGES == FIXED_EDGES) {
+        if (exA != NO_EDGE) {
+          edge_devs_lo<T, HORD>(qrow, 1, &L.edx[0][0][r], ed0);
+          if (outer) edge_devs_lo<T, HORD>(qirow, 1, &L.edx[0][0][r], ed1);
+        }
+        if (exB != NO_EDGE) {
+          edge_devs_hi<T, HORD>(qrow, 1, &L.edx[1][0][r], ed0);
+          if (outer) edge_devs_hi<T, HORD>(qirow, 1, &L.edx[1][0][r], ed1);
+        }
+      } else {
+        edge_devs<T, HORD>(exA, false, exi, edA, ed0);
+        edge_devs<T, HORD>(exB, true, exi, edB, ed0 + sb * 32);
+        if (outer) {
+          edge_devs<T, HORD>(exA, false, exo, edA, ed1);
+          edge_devs<T, HORD>(exB, true, exo, edB, ed1 + sb * 32);
+        }
       }
     }
-    const bool efw = EDGES && a.cube && a.eflux != nullptr && outer && ro < nj;
+    const bool efw = EDGES && a.cube && a.eflux != nullptr && outer && ro < nj && ro >= r0;
     if constexpr (std::is_same<T, float>::value && HORD == 8 && !FLUXES) {
       // FP32 hord 8: the inner line (q) and the outer one (q_i) of this row see
       // the same faces, so they march as one packed pair (x: inner, y: outer)
@@ -469,10 +522,8 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
       float fxx_prev = L.xf[r][0] * fr.x;
       float F_prev = (fr.y + fr.x) * L.mx[ro][0];
       if (efw && i0 == 1) a.eflux[efo + iq * (long long)n + (j0 + ro - 1)] = -F_prev;
-      // interior CTAs unroll the march fully (the line's rolling state then needs no register moves:
-      // 76 registers against 86); the edge-ring CTAs, at their 128-register cap, by two
-#pragma unroll(EDGES ? 2 : WIN)
-      for (int m = 6; m < WIN; ++m) {
+      const int fe = efw ? a.npx - i0 + 3 : -1;  // the high edge's face, if its flux is kept
+      auto column = [&](int m, bool last) {
         const int f = m - 2;
         const float xcol = lp.xa.x;  // q at window column f-1 of this row
         fr = pstep(m, L.cx[r][f - 3]);
@@ -481,8 +532,24 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
         fxx_prev = fxx;
         const float F = (fr.y + fr.x) * L.mx[ro][f - 3];
         if (outer) qirow[f - 4] = xcol * L.dpa[ro][f - 4] + (F_prev - F);
-        if (efw && i0 + f - 3 == a.npx) a.eflux[efo + efe + iq * (long long)n + (j0 + ro - 1)] = F;
+        if (EDGES == FIXED_EDGES ? last && fe == E_HI : f == fe) a.eflux[efo + efe + iq * (long long)n + (j0 + ro - 1)] = F;
         F_prev = F;
+      };
+      // Unrolled, the rolling state needs no register moves, but the code outgrows the instruction
+      // cache: interior CTAs by half the march, the ring's by three (its state's period; 6 x C192 x
+      // 127 levels x 9 tracers, substep: 5.54 ms fully unrolled, 5.32 by 11, 5.15 by 3, 5.23 by 2;
+      // interior then 5.15 fully, 5.10 by 13), ring CTAs with edges at any face, at their register
+      // cap, by two.
+      if constexpr (EDGES == FIXED_EDGES) {
+        column(6, false);
+#pragma unroll 3
+        for (int m = 7; m < E_HI; ++m) column(m, false);
+#pragma unroll
+        for (int m = E_HI; m < WIN; ++m) column(m, m == WIN - 1);
+      } else {
+        constexpr int STEPS = EDGES == ANY_EDGES ? 2 : 13;
+#pragma unroll(STEPS)
+        for (int m = 6; m < WIN; ++m) column(m, false);
       }
     } else {
       Line<T, HORD> li, lo;
@@ -532,12 +599,20 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
       auto ex = [qjcol](int m) { return qjcol[m * PQ]; };
       auto edA = [&L, c, eyA](int m) { return L.edy[0][m - eyA + 2][c + 3]; };
       auto edB = [&L, c, eyB](int m) { return L.edy[1][m - eyB + 2][c + 3]; };
-      edge_devs<T, HORD>(eyA, false, ex, edA, ed0);
-      edge_devs<T, HORD>(eyB, true, ex, edB, ed0 + sb * 32);
+      if constexpr (EDGES == FIXED_EDGES) {
+        if (eyA != NO_EDGE) edge_devs_lo<T, HORD>(qjcol, PQ, &L.edy[0][0][c + 3], ed0);
+        if (eyB != NO_EDGE) edge_devs_hi<T, HORD>(qjcol, PQ, &L.edy[1][0][c + 3], ed0);
+      } else {
+        edge_devs<T, HORD>(eyA, false, ex, edA, ed0);
+        edge_devs<T, HORD>(eyB, true, ex, edB, ed0 + sb * 32);
+      }
     }
     const int ig = i0 + c;
-    const bool valid_c = c < ni;
+    const bool valid_c = c < ni && (EDGES != FIXED_EDGES || c >= c0);
     const bool efw = EDGES && a.cube && a.eflux != nullptr && valid_c;
+    // rows of this column that the tile owns, from rlo or below rhi; its high edge's face, if its flux is kept
+    const int rlo = valid_c ? r0 : TW, rhi = valid_c ? nj : 0;
+    const int fe = efw ? a.npy - j0 + 3 : -1;
     T* qo = a.q_out + t * a.sQt + iq * a.sQq + k * a.sQk + pg.at(ig, j0);
     T* fyo = FLUXES ? a.fy_out + (long long)(k * a.nq + iq) * a.sFlux + pg.at(ig, j0) : nullptr;
     Line<T, HORD> ln;
@@ -555,10 +630,10 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
       const int ir = f - 4;  // interior row between faces f-1 and f
       if (FLUXES) {
         if (valid_c && f - 3 <= nj) fyo[(long long)(f - 3) * pg.pitch] = F;
-      } else if (ir < nj && valid_c) {
+      } else if (EDGES == FIXED_EDGES ? ir >= rlo : ir < rhi) {
         qo[(long long)ir * pg.pitch] = (S.qi[ir][c] + Fprev - F) * L.ub[ir][c];
       }
-      if (efw && j0 + f - 3 == a.npy) a.eflux[efo + 3 * efe + iq * (long long)n + (ig - 1)] = F;
+      if (EDGES == FIXED_EDGES ? f == E_HI && fe == E_HI : f == fe) a.eflux[efo + 3 * efe + iq * (long long)n + (ig - 1)] = F;
       Fprev = F;
     }
   }
@@ -573,15 +648,22 @@ __device__ __forceinline__ void advance_tracer(const AdvArgs<T>& a, SmemLevel<T>
   __syncwarp();
 }
 
-// Interior CTAs (no cube-face edge in their window) and edge CTAs run as two
-// instantiations: the edge code path costs registers the interior one does
-// not need.  Interior CTAs cover the rectangle [bx0, bx0+nbxi) x [by0,
+// Interior CTAs (no cube-face edge in their window) and edge CTAs run as
+// separate instantiations: the edge code path costs registers and instructions the interior
+// one does not need.  Bound: instruction issue (60 % of issue slots, 16 warps an SM) and, where
+// the march is unrolled, instruction fetch.  The ring's cost over an interior tile was the test for
+// an edge at every step of every line and its unrolled code; where the tile's size lets the last tiles
+// start TW cells before the edge (fixed_edges) the edges lie at window faces 3 and 29, and seven
+// steps of a line test.  With the staging by rows and one ownership test a store: ring tiles of 6 x C96
+// x 127 levels x 8 tracers 981 to 672 us, substep of 6 x C192 x 127 x 9 tracers 5.99 to 4.51 ms, of 6 x
+// C48 x 63 x 4 220 to 169 us.  Interior CTAs cover the rectangle [bx0, bx0+nbxi) x [by0,
 // by0+nbyi) of CTA tiles; edge CTAs enumerate the ring around it row by row.
 // CTA tile of a substep launch: interior CTAs cover the rectangle [bx0,
 // bx0+nbxi) x [by0, by0+nbyi) of CTA tiles; edge CTAs enumerate the ring
 // around it row by row.  Returns the tile's first cell (i0, j0) and size.
 struct TileCtx {
   int t, k, i0, j0, ni, nj, exA, exB, eyA, eyB;
+  int c0, r0;  // first column and row that the tile owns
   bool corner_block;
 };
 
@@ -614,6 +696,14 @@ __device__ __forceinline__ TileCtx tile_of(const AdvArgs<T>& a, const BlockMap& 
   }
   c.i0 = a.is + bx * TW;
   c.j0 = a.js + by * TW;
+  c.c0 = c.r0 = 0;
+  if (EDGES && bm.shift) {
+    const int i = min(c.i0, a.ie - TW + 1), j = min(c.j0, a.je - TW + 1);
+    c.c0 = c.i0 - i;
+    c.r0 = c.j0 - j;
+    c.i0 = i;
+    c.j0 = j;
+  }
   c.ni = min(TW, a.ie - c.i0 + 1);
   c.nj = min(TW, a.je - c.j0 + 1);
   // window faces of cube-face edges (x: west/east, y: south/north)
@@ -653,42 +743,33 @@ __device__ __forceinline__ void stage_level(const AdvArgs<T>& a, SmemLevel<T>& L
   const T* rarea = a.rarea + t * a.sMt;
   const T* dp1 = a.dp1 ? a.dp1 + fo : nullptr;
   T* dp2o = a.dp2 ? a.dp2 + fo : nullptr;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+  const int jhi = pg.jsd + pg.rows - 1, ihi = pg.isd + pg.pitch - 1;
+  // rows of a window from (ib, jb), one per warp and pass: copy(row, offset of the lane's value in a plane)
+  auto rows = [&](int nr, int nc, int ib, int jb, auto&& copy) {
+    if (lane >= nc) return;
+    const int i = min(max(ib + lane, pg.isd), ihi) - pg.isd;
+    for (int r = warp; r < nr; r += W) copy(r, i + (min(max(jb + r, pg.jsd), jhi) - pg.jsd) * pg.pitch);
+  };
   // ---- phase 1: raw windows
-  for (int e = threadIdx.x; e < NF * WIN; e += blockDim.x) {
-    const int f = e / WIN, w = e % WIN;
-    stage_ld(&L.cy[f][w], cy, pg, i0 - 3 + w, j0 + f);
-    stage_ld(&L.yf[f][w], yf, pg, i0 - 3 + w, j0 + f);
-  }
-  for (int e = threadIdx.x; e < WIN * NF; e += blockDim.x) {
-    const int r = e / NF, f = e % NF;
-    stage_ld(&L.cx[r][f], cx, pg, i0 + f, j0 - 3 + r);
-    stage_ld(&L.xf[r][f], xf, pg, i0 + f, j0 - 3 + r);
-  }
-  for (int e = threadIdx.x; e < TW * NF; e += blockDim.x) {
-    const int r = e / NF, f = e % NF;
-    stage_ld(&L.mx[r][f], mx, pg, i0 + f, j0 + r);
-    const int ff = e / TW, c = e % TW;
-    stage_ld(&L.my[ff][c], my, pg, i0 + c, j0 + ff);
-  }
-  for (int e = threadIdx.x; e < WIN * WIN; e += blockDim.x) {
-    const int r = e / WIN, w = e % WIN;
-    stage_ld(&L.area[r][w], area, pg, i0 - 3 + w, j0 - 3 + r);
-  }
-  if (a.ra_x || a.ra_y) {
-    for (int e = threadIdx.x; e < WIN * TW; e += blockDim.x) {
-      const int r = e / TW, c = e % TW;
-      if (a.ra_x) stage_ld(&L.rrx[r][c], a.ra_x, pg, i0 + c, j0 - 3 + r);
-      const int r2 = e / WIN, w = e % WIN;
-      if (a.ra_y) stage_ld(&L.rry[r2][w], a.ra_y, pg, i0 - 3 + w, j0 + r2);
-    }
-  }
-  if (dp1 != nullptr) {
-    for (int e = threadIdx.x; e < TW * TW; e += blockDim.x) {
-      const int r = e / TW, c = e % TW;
-      stage_ld(&L.dpa[r][c], dp1, pg, i0 + c, j0 + r);
-      stage_ld(&L.ub[r][c], rarea, pg, i0 + c, j0 + r);
-    }
-  }
+  rows(NF, WIN, i0 - 3, j0, [&](int r, int o) {
+    copy_async(&L.cy[r][lane], cy + o);
+    copy_async(&L.yf[r][lane], yf + o);
+  });
+  rows(WIN, NF, i0, j0 - 3, [&](int r, int o) {
+    copy_async(&L.cx[r][lane], cx + o);
+    copy_async(&L.xf[r][lane], xf + o);
+  });
+  rows(TW, NF, i0, j0, [&](int r, int o) { copy_async(&L.mx[r][lane], mx + o); });
+  rows(NF, TW, i0, j0, [&](int r, int o) { copy_async(&L.my[r][lane], my + o); });
+  rows(WIN, WIN, i0 - 3, j0 - 3, [&](int r, int o) { copy_async(&L.area[r][lane], area + o); });
+  if (a.ra_x) rows(WIN, TW, i0, j0 - 3, [&](int r, int o) { copy_async(&L.rrx[r][lane], a.ra_x + o); });
+  if (a.ra_y) rows(TW, WIN, i0 - 3, j0, [&](int r, int o) { copy_async(&L.rry[r][lane], a.ra_y + o); });
+  if (dp1 != nullptr)
+    rows(TW, TW, i0, j0, [&](int r, int o) {
+      copy_async(&L.dpa[r][lane], dp1 + o);
+      copy_async(&L.ub[r][lane], rarea + o);
+    });
   if (EDGES) {  // metrics of the one-sided edge values: dxa across x edges, dya across y edges
     const T* dxa = a.dxa + t * a.sMt;
     const T* dya = a.dya + t * a.sMt;
@@ -704,20 +785,19 @@ __device__ __forceinline__ void stage_level(const AdvArgs<T>& a, SmemLevel<T>& L
   stage_wait();
   __syncthreads();
   // ---- phase 2: derived values
-  for (int e = threadIdx.x; e < WIN * TW; e += blockDim.x) {
-    const int r = e / TW, c = e % TW;
-    L.rrx[r][c] = T(1) / (a.ra_x ? L.rrx[r][c] : L.area[r][c + 3] + L.xf[r][c] - L.xf[r][c + 1]);
-    const int r2 = e / WIN, w = e % WIN;
-    L.rry[r2][w] = T(1) / (a.ra_y ? L.rry[r2][w] : L.area[r2 + 3][w] + L.yf[r2][w] - L.yf[r2 + 1][w]);
+  for (int r = warp; r < WIN; r += W) {
+    if (lane < TW)
+      L.rrx[r][lane] = T(1) / (a.ra_x ? L.rrx[r][lane] : L.area[r][lane + 3] + L.xf[r][lane] - L.xf[r][lane + 1]);
+    if (r < TW) L.rry[r][lane] = T(1) / (a.ra_y ? L.rry[r][lane] : L.area[r + 3][lane] + L.yf[r][lane] - L.yf[r + 1][lane]);
   }
-  if (dp1 != nullptr) {
-    for (int e = threadIdx.x; e < TW * TW; e += blockDim.x) {
-      const int r = e / TW, c = e % TW;
+  if (dp1 != nullptr && lane < TW) {
+    const int c = lane;
+    for (int r = warp; r < TW; r += W) {
       const T d1 = L.dpa[r][c], ra = L.ub[r][c];
       const T d2 = d1 + (L.mx[r][c] - L.mx[r][c + 1] + L.my[r][c] - L.my[r + 1][c]) * ra;
       L.dpa[r][c] = d1 / ra;
       L.ub[r][c] = ra / d2;
-      if (r < nj && c < ni) {
+      if (r < nj && c < ni && (!EDGES || (r >= tc.r0 && c >= tc.c0))) {
         if (dp2o != nullptr) dp2o[pg.at(i0 + c, j0 + r)] = d2;
         if (!(d2 > T(0))) raise_error(a.err, FV3G_E_DELP);
       }
@@ -725,16 +805,14 @@ __device__ __forceinline__ void stage_level(const AdvArgs<T>& a, SmemLevel<T>& L
   }
   __syncthreads();
   // ---- phase 3: 0.5 mfx, 0.5 mfy
-  for (int e = threadIdx.x; e < TW * NF; e += blockDim.x) {
-    const int r = e / NF, f = e % NF;
-    L.mx[r][f] = T(0.5) * L.mx[r][f];
-    const int ff = e / TW, c = e % TW;
-    L.my[ff][c] = T(0.5) * L.my[ff][c];
+  for (int r = warp; r < NF; r += W) {
+    if (r < TW && lane < NF) L.mx[r][lane] = T(0.5) * L.mx[r][lane];
+    if (lane < TW) L.my[r][lane] = T(0.5) * L.my[r][lane];
   }
   __syncthreads();
 }
 
-template <typename T, int HORD, bool FLUXES, bool EDGES>
+template <typename T, int HORD, bool FLUXES, int EDGES>
 __device__ __forceinline__ void substep_body(const AdvArgs<T>& a, const BlockMap& bm) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemLevel<T>& L = *reinterpret_cast<SmemLevel<T>*>(smem_raw);
@@ -743,8 +821,8 @@ __device__ __forceinline__ void substep_body(const AdvArgs<T>& a, const BlockMap
   unsigned char* wbase = smem_raw + sizeof(SmemLevel<T>) + warp * warp_smem_bytes<T>(EDGES, two);
   SmemWarp<T>& S = *reinterpret_cast<SmemWarp<T>*>(wbase);
   T* eds = reinterpret_cast<T*>(wbase + sizeof(SmemWarp<T>));
-  const TileCtx tc = tile_of<T, EDGES>(a, bm);
-  stage_level<T, EDGES>(a, L, tc);
+  const TileCtx tc = tile_of<T, EDGES != NO_EDGES>(a, bm);
+  stage_level<T, EDGES != NO_EDGES>(a, L, tc);
   const int t = tc.t, k = tc.k, i0 = tc.i0, j0 = tc.j0, ni = tc.ni, nj = tc.nj;
   const int exA = tc.exA, exB = tc.exB, eyA = tc.eyA, eyB = tc.eyB;
   const int n = a.npx - 1;
@@ -755,7 +833,7 @@ __device__ __forceinline__ void substep_body(const AdvArgs<T>& a, const BlockMap
 
   for (int iq = warp; iq < a.nq; iq += W)
     advance_tracer<T, HORD, FLUXES, EDGES>(a, L, S, t, k, eds, iq, i0, j0, ni, nj, lane, exA, exB, eyA, eyB,
-                                           corner_block, efo, efe, two ? 16 : 8);
+                                           corner_block, tc.c0, tc.r0, efo, efe, two ? 16 : 8);
 }
 
 template <typename T, int HORD, bool FLUXES, bool EDGES>
@@ -763,14 +841,22 @@ __global__ void __launch_bounds__(320) k_substep(const AdvArgs<T> a, const Block
   substep_body<T, HORD, FLUXES, EDGES>(a, bm);
 }
 
-template <int HORD, bool FLUXES>
+template <int HORD, int EDGES>
 __global__ void __launch_bounds__(256, 2) k_substep_ring32(const AdvArgs<float> a, const BlockMap bm) {
-  substep_body<float, HORD, FLUXES, true>(a, bm);
+  substep_body<float, HORD, false, EDGES>(a, bm);
+}
+
+// The whole of a tile's cells in one direction, whose last CTA tile may start TW cells before
+// the high edge (so that the edges lie at window faces 3 and 29) without any other window seeing
+// an edge: at least 29 cells, and a last tile of three or more.
+inline bool fixed_edges(int is, int ie, int npx) {
+  const int n = ie - is + 1, last = n % TW;
+  return is == 1 && ie + 1 == npx && n >= TW + 3 && last != 1 && last != 2;
 }
 
 template <typename T, int HORD, bool FLUXES>
 static int launch_one(const AdvArgs<T>& a, int warps, cudaStream_t s) {
-  const BlockMap bm = block_map(a.is, a.ie, a.js, a.je, a.npx, a.npy, a.nested);
+  BlockMap bm = block_map(a.is, a.ie, a.js, a.je, a.npx, a.npy, a.nested);
   const int nint = bm.nbxi * bm.nbyi, nring = bm.nbx * bm.nby - nint;
   const int nt = adv_tiles(a);
   // edge-ring CTAs may run narrower (and at most ring_max_warps wide)
@@ -783,9 +869,15 @@ static int launch_one(const AdvArgs<T>& a, int warps, cudaStream_t s) {
   }
   if (nring > 0) {
     dim3 grid(nring, a.npz, nt);
-    if constexpr (sizeof(T) == 4)
-      k_substep_ring32<HORD, FLUXES><<<grid, 32 * wr, substep_smem_bytes<T>(wr, true, two), s>>>(a, bm);
-    else
+    if constexpr (sizeof(T) == 4) {
+      const size_t smem = substep_smem_bytes<T>(wr, true, two);
+      if (!a.nested && fixed_edges(a.is, a.ie, a.npx) && fixed_edges(a.js, a.je, a.npy)) {
+        bm.shift = 1;
+        k_substep_ring32<HORD, FIXED_EDGES><<<grid, 32 * wr, smem, s>>>(a, bm);
+      } else {
+        k_substep_ring32<HORD, ANY_EDGES><<<grid, 32 * wr, smem, s>>>(a, bm);
+      }
+    } else
       k_substep<T, HORD, FLUXES, true><<<grid, 32 * wr, substep_smem_bytes<T>(wr, true, two), s>>>(a, bm);
     FV3G_CUDA(cudaGetLastError());
   }
@@ -803,9 +895,13 @@ static int max_warps() {
 template <typename T, int HORD, bool FLUXES, bool EDGES>
 static cudaError_t set_smem_attr() {
   const int mx = (int)substep_smem_bytes<T>(max_warps<T>(), EDGES, true);
-  if constexpr (EDGES && sizeof(T) == 4)
-    return cudaFuncSetAttribute(k_substep_ring32<HORD, FLUXES>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  else
+  if constexpr (EDGES && sizeof(T) == 4) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_substep_ring32<HORD, ANY_EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k_substep_ring32<HORD, FIXED_EDGES>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  } else
     return cudaFuncSetAttribute(k_substep<T, HORD, FLUXES, EDGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
 }
 
