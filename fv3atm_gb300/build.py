@@ -15,8 +15,10 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-diag-suppress", "549,177"]
 # The column remap runs two fields per pass in unrolled copies of the same code; without automatic
 # multiply-add contraction (explicit fmaf stays fused) both copies round alike, so a field's result does not
-# depend on which slot of a pass it took (tracer groups of the pipelined host step remap bit for bit alike).
-FILE_FLAGS = {"fv3g_remap.cu": ["-fmad=false"], "fv3g_remap_col.cu": ["-fmad=false"]}
+# depend on which slot of a pass it took (tracer groups of the pipelined host step remap bit for bit alike).  The
+# same holds for the marching substep's rows beside edges and chunk ends and its other rows.
+FILE_FLAGS = {"fv3g_remap.cu": ["-fmad=false"], "fv3g_remap_col.cu": ["-fmad=false"],
+              **{f"fv3g_stream_h{h}.cu": ["-fmad=false"] for h in (1, 5, 8)}}
 
 
 def _nvcc() -> str:

@@ -227,16 +227,16 @@ __device__ __forceinline__ void edge_raw8(int kind, bool high, double x2, double
     ra = a0 - x0;
   } else if (kind == 1) {
     if (high) {
-      const double am = double(kT15) * x0 + double(kT11) * x1 + double(kT14) * dm1;
+      const double am = fma(kT14, dm1, fma(kT11, x1, kT15 * x0));
       rb = am - x1;
       ra = am - x0;
     } else {
-      ra = double(kT14) * dm1 + double(kT11) * (x1 - x0);
+      ra = fma(kT14, dm1, kT11 * (x1 - x0));
     }
   } else if (high) {
-    rb = double(kT11) * (x0 - x1) - double(kT14) * dm0;
+    rb = fma(-kT14, dm0, kT11 * (x0 - x1));
   } else {
-    const double ap = double(kT15) * x1 + double(kT11) * x0 - double(kT14) * dm0;
+    const double ap = fma(-kT14, dm0, fma(kT11, x0, kT15 * x1));
     rb = ap - x1;
     ra = ap - x0;
   }
@@ -247,7 +247,7 @@ __device__ __forceinline__ void edge_raw8(int kind, bool high, double x2, double
 // edge value with weights w.  One form with weights chosen by kind costs four FP64
 // instructions, as the fourth-order value alone does.
 __device__ __forceinline__ double interface4(double x2, double x1, double x0, double x3) {
-  return (7.0 / 12.0) * (x1 + x0) - (1.0 / 12.0) * (x2 + x3);
+  return fma(7.0 / 12.0, x1 + x0, (-1.0 / 12.0) * (x2 + x3));
 }
 __device__ __forceinline__ double interface_edge(int kind, double x2, double x1, double x0, double x3,
                                                  const double* w) {
@@ -738,18 +738,23 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 1) k_stream(const AdvArgs<d
 }
 
 // Strips, chunks and tracer groups of a launch.  Columns per lane: the choice
-// that sweeps fewer lanes over the tile's width (32 NC per strip),
-// two on a tie (half the shuffles and field reads per cell); it depends on the
-// width alone, so a tracer's result does not depend on the batch it runs in.
+// that sweeps fewer lanes over the tile's width (32 NC per strip), one on a tie: twice
+// the warps for the same FP64 work hide more of a row's latency and balance the SMs
+// better (one face of C48 L63 x 1 492 to 381 us a step, six C192 L127 x 9 173 to 171 ms).
+// It depends on the width alone, and the file is built without automatic contraction of
+// products and sums (the fused ones are written), so that a cell's value does not depend on the
+// chunk, and a tracer's result not on the batch, it is computed in.
 inline int stream_columns(int ni) {
   const int two = ni <= 58 ? 64 : 64 * ((ni + 55) / 56), one = ni <= 26 ? 32 : 32 * ((ni + 23) / 24);
-  return one < two ? 1 : 2;
+  return one <= two ? 1 : 2;
 }
 
 // Tracers per CTA and chunks along j, from a model of the launch: an SM holds
 // res CTAs (registers: 255 a thread; shared memory), and with w warps resident a
-// row of each takes time in proportion to w + 1.5 (the FP64 pipe shared, plus the
-// latency of a row: 83 % of the pipe used at 8 warps).  A CTA pays for staging a
+// row of each takes time in proportion to w + c (the FP64 pipe shared, plus the
+// latency of a row: c = 1.5 with two columns a lane, 83 % of the pipe used at 8 warps;
+// 3 with one, whose row is half the work; 1.5 there took 381 us, 3 to 8 325 us, for one face of
+// C48 L63 x 1).  A CTA pays for staging a
 // row what one more tracer would cost in part (1 / G), a chunk 9 rows of run-in,
 // and the launch whole waves of CTAs.  At six C192 tiles x 127 levels x 9 tracers
 // groups of 3 and 5 took 52.9 and 59.8 ms a substep, at 4 tracers groups of 4 and 2
@@ -763,7 +768,7 @@ inline StreamMap stream_map(int ni, int nj, int nq, int warps, long long planes)
   best.W = ((ni + best.ns - 1) / best.ns + 3) & ~3;
   best.ns = (ni + best.W - 1) / best.W;
   const int by_regs = 8;  // warps of an SM
-  const double c = 1.5;
+  const double c = NC == 1 ? 3.0 : 1.5;
   double least = 0.0;
   for (int g = std::min(std::min(warps, kStreamWarps), nq); g >= 1; --g) {
     const int ng = (nq + g - 1) / g, G = (nq + ng - 1) / ng;
