@@ -123,7 +123,8 @@ struct fv3g_state {
   void* cx = nullptr; void* cy = nullptr; void* mfx = nullptr; void* mfy = nullptr;  // inputs (unscaled)
   void* cxs = nullptr; void* cys = nullptr; void* mfxs = nullptr; void* mfys = nullptr;  // scaled copies
   void* xfx = nullptr; void* yfx = nullptr;
-  cudaMemPool_t pool = nullptr;  // buffers of one call (CallBufs)
+  cudaMemPool_t pool = nullptr;  // buffers of one call (CallBufs), made by the first call that needs any
+  std::once_flag pool_once;
   void* lev = nullptr; void* ew = nullptr;  // FP64: the marching substep's per-level planes and edge weights (AdvArgs)
   void* dp_eul = nullptr;
   void* area = nullptr; void* rarea = nullptr; void* dxa = nullptr; void* dya = nullptr;
@@ -631,12 +632,35 @@ int level_field_copy(fv3g_state* st, int field, const void* host, cudaStream_t s
 }
 
 // ------------------------------------------ tangent-linear and adjoint ---
+// The state's pool of call buffers.  A call's buffers are taken and given back in the order
+// of its stream, so calls on several streams and threads share it; what lies idle stays
+// mapped up to a sixteenth of the device's memory (the rest returns at the next
+// synchronisation) and goes with the state.  Mapping and unmapping them on every call took 6
+// of the 63 ms of a linearised step (6 x C96, 64 levels, 4 tracers, 6 substeps: 6.6 GB) and
+// 1.6 of the 7.7 ms of the pt, u and v remaps at 6 x C192 x 127 levels.
+void create_pool(fv3g_state* st) {
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  size_t idle = 0, total = 0;
+  if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemGetInfo(&idle, &total) != cudaSuccess ||
+      cudaMemPoolCreate(&st->pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    st->pool = nullptr;  // no pools on this device: the buffers are allocated by the call
+    return;
+  }
+  unsigned long long keep = total / 16;
+  cudaMemPoolSetAttribute(st->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 // Device buffers of one call (linearised step, field remap), given back at its end.
 struct CallBufs {
   fv3g_state* st;
   cudaStream_t s;
   std::vector<void*> p;
-  CallBufs(fv3g_state* state, cudaStream_t stream) : st(state), s(stream) {}
+  CallBufs(fv3g_state* state, cudaStream_t stream) : st(state), s(stream) {
+    std::call_once(st->pool_once, create_pool, st);
+  }
   CallBufs(const CallBufs&) = delete;
   CallBufs& operator=(const CallBufs&) = delete;
   ~CallBufs() {
@@ -663,27 +687,6 @@ struct CallBufs {
     return 0;
   }
 };
-
-// The state's pool of call buffers.  A call's buffers are taken and given back in the order
-// of its stream, so calls on several streams and threads share it; what lies idle stays
-// mapped up to a sixteenth of the device's memory (the rest returns at the next
-// synchronisation) and goes with the state.  Mapping and unmapping them on every call took 6
-// of the 63 ms of a linearised step (6 x C96, 64 levels, 4 tracers, 6 substeps: 6.6 GB) and
-// 1.6 of the 7.7 ms of the pt, u and v remaps at 6 x C192 x 127 levels.
-void create_pool(fv3g_state* st) {
-  cudaMemPoolProps props{};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  size_t idle = 0, total = 0;
-  if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemGetInfo(&idle, &total) != cudaSuccess ||
-      cudaMemPoolCreate(&st->pool, &props) != cudaSuccess) {
-    cudaGetLastError();
-    st->pool = nullptr;  // no pools on this device: the buffers are allocated by the call
-    return;
-  }
-  unsigned long long keep = total / 16;
-  cudaMemPoolSetAttribute(st->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-}
 
 // The trajectory of a linearised step: the forward substeps of the state's
 // inputs run with the production kernels, each substep's input (halo strips
@@ -886,7 +889,6 @@ int fv3g_state_create(const fv3g_state_desc* desc, fv3g_state** out) {
     return set_error(FV3G_E_ARG, "iv %d outside -1..1 (iv -2 needs per-column surface values qs)", d.iv);
   fv3g_state* st = new (std::nothrow) fv3g_state();
   if (!st) return set_error(FV3G_E_NOMEM, "host allocation failed");
-  create_pool(st);
   st->d = d;
   st->fp64 = d.precision == FV3G_FP64;
   st->esz = st->fp64 ? 8 : 4;
