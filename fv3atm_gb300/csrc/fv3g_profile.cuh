@@ -234,4 +234,9 @@ __device__ __forceinline__ Profile<T> layer_profile_f(int k, int km, T qk, T aL,
                                 inner ? q(k + 2) : qk, aL, aR, dmk, iv, floor_v);
 }
 
+// mean of the parabola (aL, aR, a6) over the fractional interval [x1, x2]
+template <typename T> __device__ __forceinline__ T pmean(T l, T r, T s6, T x1, T x2) {
+  return l + T(0.5) * (x1 + x2) * ((r - l) + s6) - s6 * ((x2 * x2 + x1 * x2 + x1 * x1) * T(1.0 / 3.0));
+}
+
 }  // namespace fv3g

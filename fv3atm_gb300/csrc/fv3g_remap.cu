@@ -34,11 +34,6 @@
 namespace fv3g {
 
 
-// mean of the parabola (aL, aR, a6) over the fractional interval [x1, x2]
-template <typename T> __device__ __forceinline__ T pmean(T l, T r, T s6, T x1, T x2) {
-  return l + T(0.5) * (x1 + x2) * ((r - l) + s6) - s6 * ((x2 * x2 + x1 * x2 + x1 * x1) * T(1.0 / 3.0));
-}
-
 // Thread-per-column form with a global scratch (the caller's fixed buffer);
 // used where the library may not allocate (fv3g_remap_columns_noalloc).
 template <typename T, int KORD>

@@ -17,6 +17,9 @@
 //     integer pipe;
 //   * the positivity test compares |bl + br| with the mean's height above the
 //     floor first: the parabola's minimum lies no lower than q - |bl + br|.
+// These forms take ordinary numbers; a column that holds others goes through the schemes
+// in their FP64 forms (general_fields), found by an integer test per value and one vote per
+// field.
 // A call's divisions (pressures, pivots, target thicknesses) take fast_rcp and
 // fast_div (fv3g_fp64.cuh), a third and a half of the FP64 instructions of an IEEE
 // division.  Measured: the remap of 6 x C96 L64 x 4 tracers, kord 4, 13.2 -> 2.4 ms
@@ -27,6 +30,7 @@
 
 #include "fv3g_fp64.cuh"
 #include "fv3g_internal.cuh"
+#include "fv3g_profile.cuh"
 #include "fv3g_remap.cuh"
 
 namespace fv3g {
@@ -34,6 +38,7 @@ namespace {
 
 constexpr int COLS = 4;   // columns (warps) per CTA: 4 FP64 columns are one 32-byte sector
 constexpr int SLOTS = 3;  // fields in the shared-memory ring
+constexpr int MAX_FIELDS = 32 * 32;  // fields of a launch: a bit of a lane's word each (general_fields)
 constexpr unsigned FULL = 0xffffffffu;
 
 // one pad element per 16 levels: blocked lane ownership hits distinct banks
@@ -90,8 +95,126 @@ __device__ __forceinline__ double limit9(double a, double qa, double qb, double 
   return mono ? (less(hi, lower) ? hi : lower) : (pos(dl) ? lower : below);
 }
 
+// Whether a's magnitude is ordinary: 2^-999 .. 2^977 (so neither zero, infinite nor NaN).
+__device__ __forceinline__ bool ordinary(double a) {
+  return (unsigned)(((__double2hiint(a) >> 20) & 0x7ff) - 24) <= 1976u;
+}
+__device__ __forceinline__ bool huge_or_nan(double a) { return (__double2hiint(a) & 0x7ff00000) >= 0x7d000000; }
+
+// The fields (bit f / 32 of lane f % 32's word) whose columns hold something else than
+// ordinary numbers -- a layer or target without thickness, infinities, NaN -- once more by
+// the schemes in their FP64 forms (fv3g_profile.cuh), whose minima and maxima take the number
+// beside a NaN; the overlaps come from the pressures one by one.  Rare, and called when no
+// column constant is held any more, so that the field loop keeps its registers; in that
+// loop the same as a branch spilled 36 to 400 bytes.  One warp.
 template <int KORD, int NPL>
-__global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const RemapArgs<double> a) {
+__device__ __noinline__ void general_fields(Col64<NPL>& S, double* Q, unsigned fields, long long qo, int col, int lane,
+                                            bool real, const RemapArgs<double>& a) {
+  const int km = a.km, kn = a.kn, u0 = lane * NPL, nc = (int)a.ncol;
+  const double floor_v = a.iv == 1 ? a.q_min : 0.0, qsv = a.qs ? a.qs[col] : 0.0, ps = S.pe1[pd(km)];
+  auto q = [Q, km](int k) -> double { return Q[pd(min(max(k, 0), km - 1))]; };
+  auto h = [&S, km](int k) -> double { return S.dp[pd(min(max(k, 0), km - 1))]; };
+  double *const cp = S.w1, *const rd = S.S1;  // kord 9: the interface system's elimination, row by row
+  __syncwarp();
+  double lo_b = 0.0, gb = 0.0;
+  if (KORD == 9 && km > 1) {
+    gb = h(km - 2) / h(km - 1);
+    lo_b = a.iv == -2 ? 0.0 : gb + 1.0;
+    if (lane == 0) {
+      const double g = h(1) / h(0);
+      double c = (g + 1.0) / g;
+      cp[0] = c;
+      rd[0] = 1.0 / g;
+      for (int u = 1; u < km; ++u) {
+        const double d = h(u - 1) / h(u), r = 1.0 / (2.0 * (1.0 + d) - c);
+        c = d * r;
+        cp[pd(u)] = c;
+        rd[pd(u)] = r;
+      }
+      rd[pd(km)] = 1.0 / ((a.iv == -2 ? 1.0 : gb) - lo_b * c);
+    }
+  }
+  for (int f = 0; f < a.nfield; ++f) {
+    if (!(__shfl_sync(FULL, fields, f & 31) >> (f >> 5) & 1)) continue;
+    const double* src = a.q_in + qo + f * a.sQq;
+    for (int k = lane; k < km; k += 32) Q[pd(k)] = src[(long long)k * a.sQk];
+    __syncwarp();
+    if (KORD == 9 && km > 1 && lane == 0) {
+      const double g = h(1) / h(0);
+      double y = ((g * (2.0 * g + 3.0)) * q(0) + q(1)) / (g + 1.0) * rd[0];
+      S.l[0] = y;
+      for (int u = 1; u < km; ++u) {
+        y = (3.0 * (q(u - 1) + h(u - 1) / h(u) * q(u)) - y) * rd[pd(u)];
+        S.l[pd(u)] = y;
+      }
+      const double r = a.iv == -2 ? qsv : ((gb * (2.0 * gb + 3.0)) * q(km - 1) + q(km - 2)) / (gb + 1.0);
+      y = (r - lo_b * y) * rd[pd(km)];
+      S.l[pd(km)] = y;
+      for (int u = km - 1; u >= 0; --u) S.l[pd(u)] = y = S.l[pd(u)] - cp[pd(u)] * y;
+    }
+    if (KORD == 4)
+      for (int k = u0; k < min(u0 + NPL, km); ++k) S.s[pd(k)] = ppm_slope_f<double>(k, km, q, h);
+    __syncwarp();
+    for (int u = u0; u < min(u0 + NPL, km + 1); ++u) {
+      double v;
+      if (km == 1) v = q(0);
+      else if (KORD == 9) v = k9_interface_f(S.l[pd(u)], u, km, a.iv, floor_v, q);
+      else
+        v = ppm_interface<double>(u, km, a.iv, qsv, u >= 1 ? S.s[pd(u - 1)] : 0.0, u < km ? S.s[pd(u)] : 0.0, q, h);
+      S.h[pd(u)] = v;
+    }
+    __syncwarp();
+    Profile<double> p[NPL];
+#pragma unroll
+    for (int j = 0; j < NPL; ++j) {
+      const int k = u0 + j;
+      if (k < km)
+        p[j] = layer_profile_f<double, KORD>(k, km, q(k), S.h[pd(k)], S.h[pd(k + 1)], KORD == 9 ? 0.0 : S.s[pd(k)],
+                                             a.iv, floor_v, q);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < NPL; ++j)
+      if (u0 + j < km) {
+        const int i = pd(u0 + j);
+        S.l[i] = p[j].l;
+        S.h[i] = p[j].r;
+        S.s[i] = p[j].s6;
+      }
+    __syncwarp();
+    auto pe2_at = [&](int k) -> double {
+      return a.pe2 != nullptr ? a.pe2[(long long)k * nc + col] : a.ak[k] + a.bk[k] * ps;
+    };
+    auto locate = [&](int k2, int& L, double& X) {
+      const double pt = pe2_at(k2);
+      L = min(k2, km - 1);
+      while (L > 0 && S.pe1[pd(L)] > pt) --L;
+      while (L < km - 1 && S.pe1[pd(L + 1)] <= pt) ++L;
+      X = (pt - S.pe1[pd(L)]) / (S.pe1[pd(L + 1)] - S.pe1[pd(L)]);
+    };
+    auto mean = [&](int L, double x1, double x2) { return pmean(S.l[pd(L)], S.h[pd(L)], S.s[pd(L)], x1, x2); };
+    for (int t = u0; t < min(u0 + NPL, kn); ++t) {
+      int Lt, Lb;
+      double Xt, Xb, out;
+      locate(t, Lt, Xt);
+      locate(t + 1, Lb, Xb);
+      if (Lb == Lt || (Lb == Lt + 1 && Xb == 0.0)) {
+        out = Xt == 0.0 && (Lb == Lt + 1 || Xb == 1.0) ? q(Lt) : mean(Lt, Xt, Lb == Lt ? Xb : 1.0);
+      } else {
+        double mass = Xt == 0.0 ? q(Lt) * h(Lt) : (h(Lt) * (1.0 - Xt)) * mean(Lt, Xt, 1.0);
+        for (int m = Lt + 1; m < Lb; ++m) mass = mass + q(m) * h(m);
+        if (Xb >= 1.0) mass = mass + q(Lb) * (h(Lb) * Xb);
+        else if (Xb > 0.0) mass = mass + (h(Lb) * Xb) * mean(Lb, 0.0, Xb);
+        out = mass * (1.0 / (a.dp2 ? a.dp2[(long long)t * nc + col] : pe2_at(t + 1) - pe2_at(t)));
+      }
+      if (real) a.q_out[qo + f * a.sQqo + (long long)t * a.sQk] = out;
+    }
+    __syncwarp();
+  }
+}
+
+template <int KORD, int NPL>
+__global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const __grid_constant__ RemapArgs<double> a) {
   constexpr int RP = ring_pitch64<NPL>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -174,6 +297,11 @@ __global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const RemapArgs<double
   // index) and p's fraction of it; Lt | Lb << 8 per target layer, bits 16 and 17:
   // the first / the last overlap is a whole layer.
   unsigned sched[NPL];
+  unsigned general = 0;  // fields for general_fields
+  bool odd = false;      // all of them
+#pragma unroll
+  for (int j = 0; j < NPL; ++j)
+    if (u0 + j < km) odd |= !ordinary(S.dp[pd(u0 + j)]);
   {
     int L0 = 0;
     double X0 = 0.0, p0 = 0.0;
@@ -192,6 +320,7 @@ __global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const RemapArgs<double
         if (t < kn) {
           const double dpk = a.dp2 ? a.dp2[(long long)t * nc + col] : p - p0;
           if (real && a.dp_out != nullptr) a.dp_out[fo + (long long)t * a.sFk] = dpk;
+          odd |= !ordinary(dpk) | huge_or_nan(X0) | huge_or_nan(X);
           const bool inside = k1 == L0 || (k1 == L0 + 1 && !nonzero(X));
           const double x2 = inside && k1 == L0 ? X : 1.0;  // the first overlap's end
           const bool whole = !nonzero(X0) && (!inside || k1 == L0 + 1 || dbits(X) == dbits(1.0));
@@ -221,6 +350,7 @@ __global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const RemapArgs<double
 
   const double floor_v = (a.iv == 1) ? a.q_min : 0.0;
   const double qsv = a.qs ? a.qs[col] : 0.0;
+  odd = __any_sync(FULL, odd | huge_or_nan(qsv) | huge_or_nan(floor_v));
   // ------------------------------------------------ the column's linear forms
   // kord 9: y_u = e1 q_a + e2 q_b + aj y_{u-1} (layers a, b = u-1, u; top row 0, 1;
   // bottom row km-1, km-2), a_u = y_u - cp a_{u+1}; mf, mb: the multipliers of the
@@ -335,6 +465,11 @@ __global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const RemapArgs<double
     for (int i = 0; i < NPL + 4; ++i) w[i] = Q[pd(min(max(u0 - 2 + i, 0), km - 1))];
 #pragma unroll
     for (int i = 0; i < NPL + 3; ++i) D[i] = w[i + 1] - w[i];
+    bool gen = odd;
+#pragma unroll
+    for (int j = 0; j < NPL; ++j) gen |= huge_or_nan(w[j + 2]);
+    gen = __any_sync(FULL, gen);
+    if (gen && lane == (f & 31)) general |= 1u << (f >> 5);
     // -------------------------------------------- interface values a[0..km]
     double st[NPL], dm[NPL];
 #pragma unroll
@@ -503,15 +638,23 @@ __global__ void __launch_bounds__(32 * COLS, 3) k_remap64(const RemapArgs<double
           for (int m = (int)(sc & 0xff) + 1; m < (int)((sc >> 8) & 0xff); ++m) mass = fma(Q[pd(m)], S.dp[pd(m)], mass);
           out = fma(mass, rdpk_of(t), out);
         }
-        if (real) q2[(long long)t * a.sQk] = out;
+        if (real && !gen) q2[(long long)t * a.sQk] = out;
       }
     }
   }
+  if (__any_sync(FULL, general != 0))
+    general_fields<KORD, NPL>(S, ring + warp * RP, general, qo, col, lane, real, a);
 }
 
 template <int KORD, int NPL>
 cudaError_t launch64(const RemapArgs<double>& a, cudaStream_t s) {
-  k_remap64<KORD, NPL><<<(unsigned)((a.ncol + COLS - 1) / COLS), 32 * COLS, smem64<NPL>(), s>>>(a);
+  RemapArgs<double> b = a;
+  for (int f = 0; f < a.nfield; f += MAX_FIELDS) {
+    b.nfield = std::min(MAX_FIELDS, a.nfield - f);
+    b.q_in = a.q_in + f * a.sQq;
+    b.q_out = a.q_out + f * a.sQqo;
+    k_remap64<KORD, NPL><<<(unsigned)((a.ncol + COLS - 1) / COLS), 32 * COLS, smem64<NPL>(), s>>>(b);
+  }
   return cudaGetLastError();
 }
 
