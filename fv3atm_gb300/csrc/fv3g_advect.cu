@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(256) k_level(const AdvArgs<double> a) {
     auto face = [p](double c, double* w1, double* w2) {
       const double m = fabs(c), w = 1.0 - m, v = m * w;
       w1[p] = w;
-      w2[p] = ((__double2hiint(w) < 0) == (c > 0.0)) ? -fabs(v) : fabs(v);
+      w2[p] = ((__double2hiint(w) < 0) == (c > 0.0)) ? negv(absv(v)) : absv(v);
     };
     face(a.cx[p], a.cx1, a.cx2);
     face(a.cy[p], a.cy1, a.cy2);

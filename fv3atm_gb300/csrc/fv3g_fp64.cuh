@@ -2,7 +2,8 @@
 // instructions run at 1/64 of the FP32 rate here (16 cycles of an SM per warp and
 // instruction), and |a|, -a, min, max and comparisons of doubles are FP64
 // instructions; the same on the high and low words runs in the integer pipe.
-// Values are taken to be numbers: where NaN matters, use the FP64 forms.
+// Values are taken to be numbers: a NaN compares by its bits.  Where one may come in, a
+// test on the high word goes beside the form, or chooses the FP64 one.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,16 +20,25 @@ __device__ __forceinline__ double negv(double a) {
 __device__ __forceinline__ double signed_as(double a, double b) {  // a >= 0 with the sign of b
   return __hiloint2double(__double2hiint(a) | (__double2hiint(b) & 0x80000000), __double2loint(a));
 }
+// a NaN as arithmetic leaves it (quiet); a value without a finite one
+__device__ __forceinline__ bool is_nan(double a) { return 2u * (unsigned)__double2hiint(a) > 0xffe00000u; }
+__device__ __forceinline__ bool inf_or_nan(double a) { return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000; }
 // of non-negative values
 __device__ __forceinline__ bool mag_less(double a, double b) { return dbits(a) < dbits(b); }
 __device__ __forceinline__ double mag_min(double a, double b) { return mag_less(a, b) ? a : b; }
 __device__ __forceinline__ double mag_max(double a, double b) { return mag_less(a, b) ? b : a; }
-// a 2^K for K = -2, -1, 1; a zero or of magnitude below 2^-1019 becomes zero
+// a 2^K for K = -2, -1, 1; zero, infinities, NaN and magnitudes below 2^-1019 as they are
 template <int K>
 __device__ __forceinline__ double scale2(double a) {
   const int hi = __double2hiint(a);
-  const bool ok = (hi & 0x7fffffff) >= 0x00400000;
-  return __hiloint2double(ok ? hi + K * 0x00100000 : 0, ok ? __double2loint(a) : 0);
+  const bool ok = 2u * (unsigned)hi - 0x00800000u < 0xff600000u;  // exponent field 4 .. 2046
+  return __hiloint2double(ok ? hi + K * 0x00100000 : hi, __double2loint(a));
+}
+// |a| / 4; zero for a NaN and below 2^-1019, 2^1022 for an infinity
+__device__ __forceinline__ double quarter_mag(double a) {
+  const int hi = __double2hiint(a);
+  const bool ok = 2u * (unsigned)hi - 0x00800000u <= 0xff600000u;
+  return __hiloint2double(ok ? (hi & 0x7fffffff) - 0x00200000 : 0, ok ? __double2loint(a) : 0);
 }
 // 1 / x to within an ulp in three FP64 instructions (an IEEE division takes about
 // eleven): an FP32 reciprocal r of the significand, then r + r (e + e^2) with e = 1 -
@@ -51,7 +61,7 @@ __device__ __forceinline__ double fast_div(double a, double b) {
   const int ex = (__double2hiint(b) >> 20) & 0x7ff;
   if ((unsigned)(ex - 24) > 2000u) return a / b;
   const double r = fast_rcp(b), q = a * r;
-  return fma(fma(negv(q), b, a), r, q);
+  return inf_or_nan(q) ? q : fma(fma(negv(q), b, a), r, q);  // (an infinite q has no residual)
 }
 // a != 0 by words (a test of the whole shifted pattern is compiled to an FP64 comparison)
 __device__ __forceinline__ bool nonzero(double a) {
@@ -69,11 +79,13 @@ __device__ __forceinline__ long long dkey(double a) {
   return k ^ ((k >> 63) & 0x7fffffffffffffffLL);
 }
 __device__ __forceinline__ bool less(double a, double b) { return dkey(a) < dkey(b); }
-// a into the range of x0 and x1
+// a into the range of x0 and x1, as fmin(fmax(a, lo), hi) has it: where a is NaN (as it is to be
+// where x0 or x1 is) the lower one, or the number of the two
 __device__ __forceinline__ double clamp_between(double a, double x0, double x1) {
   const bool up = less(x0, x1);
   const double lo = up ? x0 : x1, hi = up ? x1 : x0;
-  return less(a, lo) ? lo : less(hi, a) ? hi : a;
+  const double in = less(a, lo) ? lo : less(hi, a) ? hi : a;
+  return is_nan(a) ? (is_nan(lo) ? hi : lo) : in;
 }
 // a into the range of 0, x and y
 __device__ __forceinline__ double clamp0(double a, double x, double y) {

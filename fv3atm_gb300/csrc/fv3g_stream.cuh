@@ -131,7 +131,8 @@ __device__ __forceinline__ Vec<NC> veast(const Vec<NC>& a) {
 }
 
 // Monotonized central slopes in half increments: dm, |2 dm| and the sign; dp
-// and d are the differences to the cells before and after.
+// and d are the differences to the cells before and after.  Beside a NaN the slope is
+// zero, as the minimum of the numbers left has it.
 template <int NC>
 struct Slope {
   Vec<NC> dm, two;
@@ -141,7 +142,7 @@ struct Slope {
     for (int c = 0; c < NC; ++c) {
       const double xt = xp[c] - xm[c];
       const bool mono = (__double2hiint(dp[c]) ^ __double2hiint(d[c])) >= 0;
-      const double m = mag_min(scale2<-2>(absv(xt)), mag_min(absv(d[c]), absv(dp[c])));
+      const double m = mag_min(quarter_mag(xt), mag_min(absv(d[c]), absv(dp[c])));
       const double mag = mono ? m : 0.0;
       dm[c] = signed_as(mag, xt);
       two[c] = scale2<1>(mag);
@@ -203,11 +204,12 @@ __device__ __forceinline__ Vec<NC> upwind(const FaceC<NC>& f, const Vec<NC>& xl,
   });
 }
 
-// 2-dx filter test of a cell (hord 5: bl br < 0; hord 1: |lim_fac b0| < |bl - br|)
+// 2-dx filter test of a cell (hord 5: bl br < 0; hord 1: |lim_fac b0| < |bl - br|); none
+// beside a NaN passes
 template <int HORD>
 __device__ __forceinline__ bool filter_pass(double lim, double nl, double br, double b0) {
-  if (HORD == 1) return dbits(absv(lim * b0)) < dbits(absv(nl + br));
-  return opp(negv(nl), br);
+  if (HORD == 1) return dbits(absv(lim * b0)) < dbits(absv(nl + br)) && !is_nan(nl + br);
+  return opp(negv(nl), br) && !is_nan(nl) && !is_nan(br);
 }
 
 // a linear form of four cells
@@ -256,15 +258,18 @@ __device__ __forceinline__ double interface_edge(int kind, double x2, double x1,
   c[1] = kind == 2 ? w[1] : kind == 1 ? kD2 : kind == 3 ? kD3 : 7.0 / 12.0;
   c[2] = kind == 2 ? w[2] : kind == 1 ? kD3 : kind == 3 ? kD2 : 7.0 / 12.0;
   c[3] = kind == 2 ? w[3] : kind == 1 ? 0.0 : kind == 3 ? kD1 : -1.0 / 12.0;
-  return form4(c, x2, x1, x0, x3);
+  return form4(c, kind == 3 ? 0.0 : x2, x1, x0, kind == 1 ? 0.0 : x3);  // (0 times a NaN is one)
 }
 
-// CW84 eq. 1.10 with selects: 3 |d (bl + br)| > d^2, d = br - bl, as 3 |bl + br| > |d|
+// CW84 eq. 1.10 with selects: 3 |d (bl + br)| > d^2, d = br - bl, as 3 |bl + br| > |d|.  Where
+// bl br is NaN (bl + br is, or it is infinite beside a zero) the deviations stay.
 __device__ __forceinline__ void cw84_flat(double& bl, double& br) {
   const double d = br - bl, s = bl + br;
-  const bool big = mag_less(absv(d), absv(3.0 * s)), down = (__double2hiint(d) ^ __double2hiint(s)) < 0;
+  const bool zero = !nonzero(bl) || !nonzero(br);
+  const bool odd = 2u * (unsigned)__double2hiint(s) > 0xffe00000u - zero;
+  const bool big = mag_less(absv(d), absv(3.0 * s)) && !odd, down = (__double2hiint(d) ^ __double2hiint(s)) < 0;
   const double nl = big && down ? negv(scale2<1>(br)) : bl, nr = big && !down ? negv(scale2<1>(bl)) : br;
-  const bool flat = !opp(bl, br);
+  const bool flat = (zero || (__double2hiint(bl) ^ __double2hiint(br)) >= 0) && !odd;
   bl = flat ? 0.0 : nl;
   br = flat ? 0.0 : nr;
 }
