@@ -761,6 +761,7 @@ int lin_forward(fv3g_state* st, int q_split, cudaStream_t s, CallBufs& B, LinSte
   }
   CHECK(B.take(&a.dr, L.fn));
   CHECK(B.take(&a.r2, L.fn));
+  CHECK(B.take(&a.odd, 1));
   double** tq[] = {&L.tr.qc1, &L.tr.qc2, &L.tr.qi, &L.tr.qj, &L.tr.fx2, &L.tr.fy2,
                    &L.w.a1, &L.w.a2, &L.w.ai, &L.w.aj, &L.w.gx, &L.w.gy, &L.w.fx2, &L.w.fy2};
   for (double** b : tq) CHECK(B.take(b, L.qn));
@@ -1149,7 +1150,7 @@ int fv3g_state_step_tl(fv3g_state* st, int q_split, int parts, const double* dq_
   if (st->d.kord == 4) {
     FV3G_CUDA(cudaMemsetAsync(dq1, 0, sizeof(double) * L.qn, s));
     CHECK(lin_remap_tl4(L.q[L.nsplt], dq0, L.dp[L.nsplt], st->ak, st->bk, dq1, st->pg, st->plane, st->n, st->nt, st->nq,
-                        st->npz, st->npz, st->d.iv, st->d.q_min, s));
+                        st->npz, st->npz, st->d.iv, st->d.q_min, L.a.odd, s));
     CHECK(lin_user_copy(st, dq1, dq_out, true, s));
     FV3G_CUDA(cudaStreamSynchronize(s));
     return 0;
@@ -1214,7 +1215,7 @@ int fv3g_state_step_ad(fv3g_state* st, int q_split, int parts, const double* q_a
   if (parts & 2) {
     CHECK(lin_user_copy(st, g, q_ad_out, false, s));
     CHECK(lin_remap_ad(L.q[L.nsplt], L.dp[L.nsplt], st->ak, st->bk, g, a0, st->pg, st->plane, st->n, st->nt, st->nq,
-                       st->npz, st->npz, st->d.iv, st->d.q_min, st->d.kord, s));
+                       st->npz, st->npz, st->d.iv, st->d.q_min, st->d.kord, L.a.odd, s));
   } else {
     CHECK(lin_user_copy(st, a0, q_ad_out, false, s));
   }

@@ -167,10 +167,18 @@ __device__ __forceinline__ bool edge_face(int f, int eLo, int eHi) {
 // runs at 1/64 of the FP32 rate, so the count of FP64 operations is the cost:
 // six C96 tiles x 64 levels x 4 tracers, hord 5, six substeps took 505 ms in
 // both kernels with six passes per face.  The branch conventions are those of
-// ppm_face on dual numbers (on a tie the later operand).
+// ppm_face on dual numbers (on a tie the later operand); faces with an infinity or a NaN in their
+// window are reported in odd and left to k_lin_odd.
 __device__ __forceinline__ void put_weights(double* w, long long ws, const double* W) {
 #pragma unroll
   for (int s = 0; s < 6; ++s) w[s * ws] = W[s];
+}
+
+__device__ __forceinline__ bool odd_window(const double* x, double c) {
+  bool odd = inf_or_nan(c);
+#pragma unroll
+  for (int s = 0; s < 6; ++s) odd |= inf_or_nan(x[s]);
+  return odd;
 }
 
 // Slope of the middle cell of (xm, x0, xp) and its derivatives p on the three.
@@ -195,10 +203,11 @@ __device__ __forceinline__ double slope_grad(double xm, double x0, double xp, do
 
 template <class XV>
 __device__ __forceinline__ double face_weights(int hord, double lim_fac, int f, const XV& xv, double c, double* w,
-                                               long long ws) {
+                                               long long ws, int* odd) {
   double x[6], W[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int s = 0; s < 6; ++s) x[s] = xv(f - 3 + s);
+  if (odd_window(x, c)) *odd = 1;
   const bool left = pos(c);  // upwind cell f-1 (window cell 2), else f (window cell 3)
   const double ac = absv(c), w1 = 1.0 - ac, w2 = ac * w1;
   const double wd = w1 - w2, nw2 = negv(w2);
@@ -256,23 +265,27 @@ __device__ __forceinline__ double face_weights(int hord, double lim_fac, int f, 
 // one-sided ones included.  hord 8: one forward-mode pass of ppm_face per
 // cell (six faces of a line).
 template <class XV, class DF>
-__device__ double edge_face_weights(int hord, double lim_fac, int f, const XV& xv, const DF& DX, double c, int eLo,
-                                    int eHi, double* w, long long ws) {
-  if (hord == 8) {
-    double val = 0.0;
+__device__ __forceinline__ double forward_weights(int hord, double lim_fac, int f, const XV& xv, const DF& DX, double c,
+                                                  int eLo, int eHi, double* w, long long ws) {
+  double val = 0.0;
 #pragma unroll 1
-    for (int s = 0; s < 6; ++s) {
-      const int ms = f - 3 + s;
-      auto X = [&](int m) -> D2 { return D2(xv(m), m == ms ? 1.0 : 0.0); };
-      const D2 r = ppm_face<D2>(hord, lim_fac, f, X, DX, c, eLo, eHi);
-      w[s * ws] = r.d;
-      val = r.v;
-    }
-    return val;
+  for (int s = 0; s < 6; ++s) {
+    const int ms = f - 3 + s;
+    auto X = [&](int m) -> D2 { return D2(xv(m), m == ms ? 1.0 : 0.0); };
+    const D2 r = ppm_face<D2>(hord, lim_fac, f, X, DX, c, eLo, eHi);
+    w[s * ws] = r.d;
+    val = r.v;
   }
+  return val;
+}
+template <class XV, class DF>
+__device__ double edge_face_weights(int hord, double lim_fac, int f, const XV& xv, const DF& DX, double c, int eLo,
+                                    int eHi, double* w, long long ws, int* odd) {
+  if (hord == 8) return forward_weights(hord, lim_fac, f, xv, DX, c, eLo, eHi, w, ws);
   double x[6];
 #pragma unroll
   for (int s = 0; s < 6; ++s) x[s] = xv(f - 3 + s);
+  if (odd_window(x, c)) *odd = 1;
   double G[3][6], al[3];  // taps on the window and values of interfaces f-1, f, f+1
 #pragma unroll
   for (int g = 0; g < 3; ++g) {
@@ -443,7 +456,7 @@ __global__ void k_lin_inner(const LinArgs a, const LinTraj tr) {
     const double* line = tr.qc2 + c.q0;
     auto xv = [&](int m) { return line[pg.at(c.i, m)]; };
     tr.fy2[c.q0 + c.p] =
-        face_weights(a.hord, a.lim_fac, c.j, xv, a.cy[c.lev + c.p], tr.wyi + c.q0 + c.p, ws);
+        face_weights(a.hord, a.lim_fac, c.j, xv, a.cy[c.lev + c.p], tr.wyi + c.q0 + c.p, ws, a.odd);
   }
   if (!xi_face(a, c.i, c.j)) {
     for (int s = 0; s < 6; ++s) tr.wxi[s * ws + c.q0 + c.p] = 0.0;
@@ -452,7 +465,7 @@ __global__ void k_lin_inner(const LinArgs a, const LinTraj tr) {
     const double* line = tr.qc1 + c.q0;
     auto xv = [&](int m) { return line[pg.at(m, c.j)]; };
     tr.fx2[c.q0 + c.p] =
-        face_weights(a.hord, a.lim_fac, c.i, xv, a.cx[c.lev + c.p], tr.wxi + c.q0 + c.p, ws);
+        face_weights(a.hord, a.lim_fac, c.i, xv, a.cx[c.lev + c.p], tr.wxi + c.q0 + c.p, ws, a.odd);
   }
 }
 
@@ -486,8 +499,38 @@ __global__ void k_lin_edges(const LinArgs a, const LinTraj tr, int outer) {
   auto at = [&](int m) { return ydir ? pg.at(line, m) : pg.at(m, line); };
   auto xv = [&](int m) { return src[at(m)]; };
   auto dx = [&](int m) { return da[at(m)]; };
-  const double fl = edge_face_weights(a.hord, a.lim_fac, f, xv, dx, (ydir ? a.cy : a.cx)[lev + p], eLo, eHi, w, ws);
+  const double fl = edge_face_weights(a.hord, a.lim_fac, f, xv, dx, (ydir ? a.cy : a.cx)[lev + p], eLo, eHi, w, ws,
+                                      a.odd);
   if (!outer) (ydir ? tr.fy2 : tr.fx2)[q0 + p] = fl;
+}
+
+// Faces with an infinity or a NaN in their window or Courant number: the same by forward-mode
+// passes, after the kernels of a pass reported one in a.odd (else this ends at once: 12
+// launches in a step of six substeps).
+__global__ void __launch_bounds__(128) k_lin_odd(const LinArgs a, const LinTraj tr, int outer) {
+  if (*a.odd == 0) return;
+  const PlaneGeom& pg = a.pg;
+  const long long ws = (long long)a.nt * a.nq * a.npz * a.P, n = 2 * ws;
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    const bool ydir = e >= ws;
+    const long long id = ydir ? e - ws : e, p = id % a.P, pl = id / a.P, q0 = pl * a.P;
+    const int per_tile = a.nq * a.npz, t = (int)(pl / per_tile);
+    const long long lev = ((long long)t * a.npz + pl % a.npz) * a.P, met = (long long)t * a.P;
+    const int i = pg.isd + (int)(p % pg.pitch), j = pg.jsd + (int)(p / pg.pitch);
+    if (!(ydir ? (outer ? yo_face(a, i, j) : yi_face(a, i, j)) : (outer ? xo_face(a, i, j) : xi_face(a, i, j)))) continue;
+    const double* src = (outer ? (ydir ? tr.qj : tr.qi) : (ydir ? tr.qc2 : tr.qc1)) + q0;
+    const double* da = (ydir ? a.dya : a.dxa) + met;
+    const double c = (ydir ? a.cy : a.cx)[lev + p];
+    const int f = ydir ? j : i;
+    auto xv = [&](int m) { return src[ydir ? pg.at(i, m) : pg.at(m, j)]; };
+    auto dx = [&](int m) { return da[ydir ? pg.at(i, m) : pg.at(m, j)]; };
+    double x[6];
+    for (int s = 0; s < 6; ++s) x[s] = xv(f - 3 + s);
+    if (!odd_window(x, c)) continue;
+    double* w = (outer ? (ydir ? tr.wyo : tr.wxo) : (ydir ? tr.wyi : tr.wxi)) + q0 + p;
+    const double fl = forward_weights(a.hord, a.lim_fac, f, xv, dx, c, ydir ? a.es : a.ew, ydir ? a.en : a.ee, w, ws);
+    if (!outer) (ydir ? tr.fy2 : tr.fx2)[q0 + p] = fl;
+  }
 }
 
 // Inner updates: q_i = (q area + yfx fy2 - yfx' fy2') / ra_y on the compute
@@ -526,14 +569,14 @@ __global__ void k_lin_outer(const LinArgs a, const LinTraj tr) {
   } else if (!edge_face(c.i, a.ew, a.ee)) {
     const double* line = tr.qi + c.q0;
     auto xv = [&](int m) { return line[pg.at(m, c.j)]; };
-    face_weights(a.hord, a.lim_fac, c.i, xv, a.cx[c.lev + c.p], tr.wxo + c.q0 + c.p, ws);
+    face_weights(a.hord, a.lim_fac, c.i, xv, a.cx[c.lev + c.p], tr.wxo + c.q0 + c.p, ws, a.odd);
   }
   if (!yo_face(a, c.i, c.j)) {
     for (int s = 0; s < 6; ++s) tr.wyo[s * ws + c.q0 + c.p] = 0.0;
   } else if (!edge_face(c.j, a.es, a.en)) {
     const double* line = tr.qj + c.q0;
     auto xv = [&](int m) { return line[pg.at(c.i, m)]; };
-    face_weights(a.hord, a.lim_fac, c.j, xv, a.cy[c.lev + c.p], tr.wyo + c.q0 + c.p, ws);
+    face_weights(a.hord, a.lim_fac, c.j, xv, a.cy[c.lev + c.p], tr.wyo + c.q0 + c.p, ws, a.odd);
   }
 }
 
@@ -789,6 +832,7 @@ dim3 plane_grid(const LinArgs& a) {
 // One column's source means, slopes, interfaces, the overlap schedule and
 // the adjoints, in local memory.
 struct ColumnAd {
+  static constexpr bool DUAL = false;
   double q[KMAX], h[KMAX], d[KMAX], a[KMAX + 1];
   double qa[KMAX], da[KMAX], aa[KMAX + 1];
   double pl[KMAX], pr[KMAX], p6[KMAX];  // adjoints of the layer parabolas (left, right edge, curvature)
@@ -805,6 +849,8 @@ __device__ __forceinline__ void pmean_grad(double x1, double x2, double g, doubl
   g6 += g * (m - (x2 * x2 + x1 * x2 + x1 * x1) * (1.0 / 3.0));
 }
 
+constexpr double kNaN = __builtin_nan("");
+
 // ---- local derivatives of the kord-4 scheme (fv3g_profile.cuh) at the trajectory,
 // every branch frozen; on a tie the later operand, as min, max and the tests on
 // dual numbers take it.  The columns are bound by FP64 instructions and their per-thread
@@ -812,10 +858,24 @@ __device__ __forceinline__ void pmean_grad(double x1, double x2, double g, doubl
 // for six C96 tiles x 64 levels x 4 tracers, these 6.5 ms (reverse) and, instead of the
 // column kernel on dual numbers, 6.2 ms (tangent; 12.0 ms).
 
+// slope4_grad with an infinity or a NaN among the means, in forward mode.
+template <bool DUAL>
+__device__ __noinline__ double slope4_odd(double qm, double q0, double qp, double d0, double d1, double d2, double* p) {
+  D2 r;
+  for (int s = 0; s < 3; ++s) {
+    r = ppm_slope(D2(qm, s == 0 ? 1.0 : 0.0), D2(q0, s == 1 ? 1.0 : 0.0), D2(qp, s == 2 ? 1.0 : 0.0), D2(d0), D2(d1), D2(d2));
+    p[s] = r.d;
+  }
+  return DUAL ? r.v : ppm_slope<double>(qm, q0, qp, d0, d1, d2);
+}
 // d slope / d (qm, q0, qp) and the slope of a layer from the means and thicknesses of
-// the layer and its neighbours.
+// the layer and its neighbours.  DUAL: beside an infinity or a NaN the value is that of the dual
+// numbers (the tangent's columns), whose comparisons choose otherwise than fmin and fmax.
+// ODD, here and below: the column may hold infinities or NaN (a kernel of its own for those).
+template <bool ODD, bool DUAL = false>
 __device__ __forceinline__ double slope4_grad(double qm, double q0, double qp, double d0, double d1, double d2,
                                               double* p) {
+  if (ODD && (inf_or_nan(qm) || inf_or_nan(q0) || inf_or_nan(qp))) return slope4_odd<DUAL>(qm, q0, qp, d0, d1, d2, p);
   const double f = d1 * fast_rcp(d0 + d1 + d2);
   const double A = f * ((2.0 * d0 + d1) * fast_rcp(d2 + d1)), B = f * ((d1 + 2.0 * d2) * fast_rcp(d0 + d1));
   const double Dm = q0 - qm, Dp = qp - q0, s = qp - qm;
@@ -852,10 +912,37 @@ struct InterfaceDer {
   int lo;
   bool inner;
 };
+__device__ __forceinline__ bool inner_interface(int u, int km) { return km > 2 && u >= 2 && u <= km - 2; }
+// an infinity or a NaN in what interface u reads (dml, dmr: the slopes of layers u-1, u)
+template <class QF>
+__device__ __forceinline__ bool odd_interface(int u, int km, const QF& q, double dml, double dmr) {
+  if (inner_interface(u, km)) return inf_or_nan(q(u - 1)) || inf_or_nan(q(u)) || inf_or_nan(dml) || inf_or_nan(dmr);
+  const int lo = u <= 1 ? 0 : km - 3;
+  return inf_or_nan(q(lo)) || inf_or_nan(q(lo + 1)) || inf_or_nan(q(lo + 2));
+}
+// its derivatives in forward mode
 template <class QF, class HF>
-__device__ InterfaceDer interface_der(int u, int km, int iv, const QF& q, const HF& h) {
+__device__ __noinline__ InterfaceDer interface_odd(int u, int km, int iv, QF q, HF h, double dml, double dmr) {
+  InterfaceDer D{{0.0, 0.0, 0.0}, 0.0, 0.0, 0, inner_interface(u, km)};
+  D.lo = D.inner ? u - 1 : u <= 1 || km == 2 ? 0 : km - 3;
+  enum { SLOPE_L = 1000, SLOPE_R };  // seeds beside the means' 0..2
+  auto pass = [&](int s) -> double {
+    auto qd = [&](int k) -> D2 { return D2(q(k), min(max(k, 0), km - 1) == D.lo + s ? 1.0 : 0.0); };
+    auto hd = [&](int k) -> D2 { return D2(h(k)); };
+    return ppm_interface<D2>(u, km, iv, D2(0.0), D2(dml, s == SLOPE_L ? 1.0 : 0.0), D2(dmr, s == SLOPE_R ? 1.0 : 0.0), qd, hd).d;
+  };
+  for (int s = 0; s < (D.inner || km == 2 ? 2 : 3); ++s) D.q[s] = pass(s);
+  if (D.inner) {
+    D.dl = pass(SLOPE_L);
+    D.dr = pass(SLOPE_R);
+  }
+  return D;
+}
+template <bool ODD, class QF, class HF>
+__device__ InterfaceDer interface_der(int u, int km, int iv, const QF& q, const HF& h, double dml, double dmr) {
+  if (ODD && odd_interface(u, km, q, dml, dmr)) return interface_odd(u, km, iv, q, h, dml, dmr);
   InterfaceDer D{{0.0, 0.0, 0.0}, 0.0, 0.0, 0, false};
-  if (km > 2 && u >= 2 && u <= km - 2) {
+  if (inner_interface(u, km)) {
     const double hm = h(u - 2), h0 = h(u - 1), h1 = h(u), h2 = h(u + 1);
     const double pair = fast_rcp(h0 + h1), sall = fast_rcp(hm + h0 + h1 + h2);
     const double fa = (hm + h0) * fast_rcp(2.0 * h0 + h1), fb = (h2 + h1) * fast_rcp(2.0 * h1 + h0);
@@ -911,14 +998,20 @@ __device__ InterfaceDer interface_der(int u, int km, int iv, const QF& q, const 
 }
 
 // d bl, d br of a layer's limited edge deviations: l[0] (d aL - d q) + l[1] (d aR - d
-// q) + l[2] d slope, r likewise; low: the positivity scaling acts (layer_der_low).
+// q) + l[2] d slope, r likewise; low: the positivity scaling acts, or an infinity or a NaN
+// comes in (layer_der_low).
 struct LayerDer {
   double l[3], r[3];
   bool low;
 };
+template <bool ODD>
 __device__ __forceinline__ LayerDer layer_der(bool inner, double q, double aL, double aR, double d, int iv,
                                               double floor_v) {
   LayerDer D{{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, false};
+  if (ODD && (inf_or_nan(q) || inf_or_nan(aL) || inf_or_nan(aR) || inf_or_nan(d))) {
+    D.low = true;
+    return D;
+  }
   const double b0 = aL - q, r0 = aR - q;
   double bl, br;
   if (inner) {  // Lin (2004): at most |2 d| with the sign of d
@@ -959,9 +1052,11 @@ __device__ __forceinline__ LayerDer layer_der(bool inner, double q, double aL, d
   }
   return D;
 }
-// The layer's (l, r, s6) by (q, aL, aR, d) in forward mode: layers near the floor.
-__device__ __noinline__ void layer_der_low(int k, int km, double q, double aL, double aR, double d, int iv,
+// The layer's (l, r, s6) by (q, aL, aR, d) in forward mode: layers near the floor, or beside a NaN.
+// Returns whether the parabola's values (as its mean takes them) are finite.
+__device__ __noinline__ bool layer_der_low(int k, int km, double q, double aL, double aR, double d, int iv,
                                            double floor_v, double (*J)[4]) {
+  bool finite = true;
   for (int s = 0; s < 4; ++s) {
     const D2 qd(q, s == 0 ? 1.0 : 0.0);
     const Profile<D2> P = layer_profile<D2, 4>(k, km, qd, qd, qd, qd, qd, D2(aL, s == 1 ? 1.0 : 0.0),
@@ -969,29 +1064,42 @@ __device__ __noinline__ void layer_der_low(int k, int km, double q, double aL, d
     J[0][s] = P.l.d;
     J[1][s] = P.r.d;
     J[2][s] = P.s6.d;
+    finite = !inf_or_nan(P.s6.v) && !inf_or_nan((P.r.v - P.l.v) + P.s6.v);
   }
+  return finite;
 }
 
 // Slopes C.d and interface values C.a of the trajectory (C.q, C.h).
-template <class CC, class QF, class HF>
+template <bool ODD, class CC, class QF, class HF>
 __device__ void column_forward4(CC& C, int km, int iv, double qs, const QF& qf, const HF& hf) {
   double p[3];
   for (int k = 0; k < km; ++k)
-    C.d[k] = k < 1 || k > km - 2 ? 0.0 : slope4_grad(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], p);
+    C.d[k] = k < 1 || k > km - 2 ? 0.0 : slope4_grad<ODD, CC::DUAL>(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], p);
   for (int u = 0; u <= km; ++u) {
-    if (km > 2 && u >= 2 && u <= km - 2) {
-      const InterfaceDer D = interface_der(u, km, iv, qf, hf);
+    const double dml = u >= 1 ? C.d[u - 1] : 0.0, dmr = u < km ? C.d[u] : 0.0;
+    if (inner_interface(u, km) && !(ODD && odd_interface(u, km, qf, dml, dmr))) {
+      const InterfaceDer D = interface_der<false>(u, km, iv, qf, hf, dml, dmr);
       C.a[u] = fma(D.q[1], C.q[u] - C.q[u - 1], C.q[u - 1]) + fma(D.dr, C.d[u], D.dl * C.d[u - 1]);
+    } else if (ODD && CC::DUAL) {
+      auto qd = [&](int k) -> D2 { return D2(qf(k)); };
+      auto hd = [&](int k) -> D2 { return D2(hf(k)); };
+      C.a[u] = ppm_interface<D2>(u, km, iv, D2(qs), D2(dml), D2(dmr), qd, hd).v;
     } else {
-      C.a[u] = ppm_interface<double>(u, km, iv, qs, 0.0, 0.0, qf, hf);
+      C.a[u] = ppm_interface<double>(u, km, iv, qs, dml, dmr, qf, hf);
     }
   }
+}
+
+__device__ __forceinline__ bool odd_column(const double* q, int km) {
+  bool odd = false;
+  for (int k = 0; k < km; ++k) odd |= inf_or_nan(q[k]);
+  return odd;
 }
 
 // Reverse of one column: pe1(k) (k = 0..km) source interface pressures,
 // pe2(k) target ones, G2(k2) the target adjoints; leaves the source
 // adjoints in C.qa.  C.q holds the source means.
-template <class PE1, class PE2, class G2>
+template <bool ODD, class PE1, class PE2, class G2>
 __device__ void column_ad4(ColumnAd& C, int km, int kn, int iv, double floor_v, double qs, const PE1& pe1,
                            const PE2& pe2, const G2& g2) {
   // thicknesses and the overlap schedule, as the forward kernel forms them
@@ -1017,7 +1125,7 @@ __device__ void column_ad4(ColumnAd& C, int km, int kn, int iv, double floor_v, 
   }
   auto qf = [&](int k) -> double { return C.q[min(max(k, 0), km - 1)]; };
   auto hf = [&](int k) -> double { return C.h[min(max(k, 0), km - 1)]; };
-  column_forward4(C, km, iv, qs, qf, hf);
+  column_forward4<ODD>(C, km, iv, qs, qf, hf);
   for (int k = 0; k < km; ++k) C.qa[k] = C.da[k] = C.pl[k] = C.pr[k] = C.p6[k] = 0.0;
   for (int u = 0; u <= km; ++u) C.aa[u] = 0.0;
 
@@ -1048,7 +1156,7 @@ __device__ void column_ad4(ColumnAd& C, int km, int kn, int iv, double floor_v, 
   for (int k = 0; k < km; ++k) {
     const double pl = C.pl[k], pr = C.pr[k], p6 = C.p6[k];
     if (pl == 0.0 && pr == 0.0 && p6 == 0.0) continue;
-    const LayerDer D = layer_der(k >= 2 && k <= km - 3, C.q[k], C.a[k], C.a[k + 1], C.d[k], iv, floor_v);
+    const LayerDer D = layer_der<ODD>(k >= 2 && k <= km - 3, C.q[k], C.a[k], C.a[k + 1], C.d[k], iv, floor_v);
     double gL, gR, gd, gq = pl + pr;
     if (!D.low) {
       const double gl = fma(-3.0, p6, pl), gr = fma(-3.0, p6, pr);
@@ -1073,7 +1181,7 @@ __device__ void column_ad4(ColumnAd& C, int km, int kn, int iv, double floor_v, 
   for (int u = 0; u <= km; ++u) {
     const double g = C.aa[u];
     if (g == 0.0) continue;
-    const InterfaceDer D = interface_der(u, km, iv, qf, hf);
+    const InterfaceDer D = interface_der<ODD>(u, km, iv, qf, hf, u >= 1 ? C.d[u - 1] : 0.0, u < km ? C.d[u] : 0.0);
     for (int s = 0; s < 3; ++s)
       if (D.q[s] != 0.0) C.qa[D.lo + s] += D.q[s] * g;
     if (D.inner) {
@@ -1086,7 +1194,7 @@ __device__ void column_ad4(ColumnAd& C, int km, int kn, int iv, double floor_v, 
     const double g = C.da[k];
     if (g == 0.0) continue;
     double p[3];
-    slope4_grad(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], p);
+    slope4_grad<ODD>(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], p);
     for (int s = 0; s < 3; ++s) C.qa[k - 1 + s] = fma(p[s], g, C.qa[k - 1 + s]);
   }
 }
@@ -1094,10 +1202,12 @@ __device__ void column_ad4(ColumnAd& C, int km, int kn, int iv, double floor_v, 
 // Every interior column and tracer of the state (thread per column and
 // tracer): pressures from ptop = ak[0] and the running sum of dp, targets
 // ak + bk ps.
+template <bool ODD>
 __global__ void __launch_bounds__(64) k_remap_ad_state(const double* q, const double* dp, const double* ak,
                                                        const double* bk, const double* q2_ad, double* q_ad,
                                                        PlaneGeom pg, long long P, int n, int nt, int nq, int km,
-                                                       int kn, int iv, double floor_v) {
+                                                       int kn, int iv, double floor_v, int* odd) {
+  if (ODD && *odd == 0) return;
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long ncol = (long long)nt * n * n;
   if (id >= ncol * nq) return;
@@ -1110,6 +1220,10 @@ __global__ void __launch_bounds__(64) k_remap_ad_state(const double* q, const do
   ColumnAd C;
   const long long qb = ((long long)t * nq + iq) * km * P + p;
   for (int k = 0; k < km; ++k) C.q[k] = q[qb + (long long)k * P];
+  if (odd_column(C.q, km) != ODD) {
+    if (!ODD) *odd = 1;
+    return;
+  }
   const double* dpc = dp + (long long)t * km * P + p;
   double ps = ak[0];
   for (int k = 0; k < km; ++k) ps += dpc[(long long)k * P];
@@ -1121,21 +1235,24 @@ __global__ void __launch_bounds__(64) k_remap_ad_state(const double* q, const do
   auto pe2 = [&](int k) { return ak[k] + bk[k] * ps; };
   const long long ob = ((long long)t * nq + iq) * kn * P + p;
   auto g2 = [&](int k2) { return q2_ad[ob + (long long)k2 * P]; };
-  column_ad4(C, km, kn, iv, floor_v, 0.0, pe1, pe2, g2);
+  column_ad4<ODD>(C, km, kn, iv, floor_v, 0.0, pe1, pe2, g2);
   for (int k = 0; k < km; ++k) q_ad[qb + (long long)k * P] = C.qa[k];
 }
 
 // Tangent-linear of the same columns: the tangents of the slopes, interfaces and
 // layers from their closed-form derivatives, integrated over the overlaps.
 struct ColumnTl {
+  static constexpr bool DUAL = true;
   double q[KMAX], h[KMAX], d[KMAX], a[KMAX + 1];
   double t[KMAX], td[KMAX], ta[KMAX + 1];  // tangents of the means, slopes and interfaces
   double tl[KMAX], tr[KMAX], t6[KMAX];     // and of the layer parabolas
 };
+template <bool ODD>
 __global__ void __launch_bounds__(64) k_remap_tl4_state(const double* q, const double* dq, const double* dp,
                                                         const double* ak, const double* bk, double* dq2, PlaneGeom pg,
                                                         long long P, int n, int nt, int nq, int km, int kn, int iv,
-                                                        double floor_v) {
+                                                        double floor_v, int* odd) {
+  if (ODD && *odd == 0) return;
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long ncol = (long long)nt * n * n;
   if (id >= ncol * nq) return;
@@ -1155,46 +1272,57 @@ __global__ void __launch_bounds__(64) k_remap_tl4_state(const double* q, const d
     C.h[k] = next - ps;  // as the forward kernel: differences of the running pressure
     ps = next;
   }
+  if (odd_column(C.q, km) != ODD) {
+    if (!ODD) *odd = 1;
+    return;
+  }
   auto qf = [&](int k) -> double { return C.q[min(max(k, 0), km - 1)]; };
   auto hf = [&](int k) -> double { return C.h[min(max(k, 0), km - 1)]; };
-  column_forward4(C, km, iv, 0.0, qf, hf);
+  column_forward4<ODD>(C, km, iv, 0.0, qf, hf);
   for (int k = 0; k < km; ++k) {
     double g[3], v = 0.0;
     if (k >= 1 && k <= km - 2) {
-      slope4_grad(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], g);
+      slope4_grad<ODD, true>(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], g);
       v = fma(g[0], C.t[k - 1], fma(g[1], C.t[k], g[2] * C.t[k + 1]));
     }
     C.td[k] = v;
   }
   for (int u = 0; u <= km; ++u) {
-    const InterfaceDer D = interface_der(u, km, iv, qf, hf);
+    const InterfaceDer D = interface_der<ODD>(u, km, iv, qf, hf, u >= 1 ? C.d[u - 1] : 0.0, u < km ? C.d[u] : 0.0);
     double v = 0.0;
     for (int s = 0; s < 3; ++s)
       if (D.q[s] != 0.0) v = fma(D.q[s], C.t[D.lo + s], v);
     if (D.inner) v += fma(D.dl, C.td[u - 1], D.dr * C.td[u]);
     C.ta[u] = v;
   }
+  // a tangent that a branch leaves out (coefficient zero) may be NaN
+  auto term = [](double c, double x) -> double { return nonzero(c) ? c * x : 0.0; };
   for (int k = 0; k < km; ++k) {
-    const LayerDer D = layer_der(k >= 2 && k <= km - 3, C.q[k], C.a[k], C.a[k + 1], C.d[k], iv, floor_v);
+    const LayerDer D = layer_der<ODD>(k >= 2 && k <= km - 3, C.q[k], C.a[k], C.a[k + 1], C.d[k], iv, floor_v);
     if (!D.low) {
       const double eL = C.ta[k] - C.t[k], eR = C.ta[k + 1] - C.t[k];
-      const double bl = D.l[0] * eL + D.l[1] * eR + D.l[2] * C.td[k], br = D.r[0] * eL + D.r[1] * eR + D.r[2] * C.td[k];
+      double bl = D.l[0] * eL + D.l[1] * eR + D.l[2] * C.td[k], br = D.r[0] * eL + D.r[1] * eR + D.r[2] * C.td[k];
+      if (ODD) {
+        bl = term(D.l[0], eL) + term(D.l[1], eR) + term(D.l[2], C.td[k]);
+        br = term(D.r[0], eL) + term(D.r[1], eR) + term(D.r[2], C.td[k]);
+      }
       C.tl[k] = C.t[k] + bl;
       C.tr[k] = C.t[k] + br;
       C.t6[k] = -3.0 * (bl + br);
     } else {
       double J[3][4];
-      layer_der_low(k, km, C.q[k], C.a[k], C.a[k + 1], C.d[k], iv, floor_v, J);
+      const bool finite = layer_der_low(k, km, C.q[k], C.a[k], C.a[k + 1], C.d[k], iv, floor_v, J);
       const double in[4] = {C.t[k], C.ta[k], C.ta[k + 1], C.td[k]};
       double o[3] = {0.0, 0.0, 0.0};
       for (int r = 0; r < 3; ++r)
-        for (int s = 0; s < 4; ++s) o[r] += J[r][s] * in[s];
-      C.tl[k] = o[0];
-      C.tr[k] = o[1];
-      C.t6[k] = o[2];
+        for (int s = 0; s < 4; ++s) o[r] += ODD ? term(J[r][s], in[s]) : J[r][s] * in[s];
+      C.tl[k] = !ODD || finite ? o[0] : kNaN;
+      C.tr[k] = !ODD || finite ? o[1] : kNaN;
+      C.t6[k] = !ODD || finite ? o[2] : kNaN;
     }
   }
-  // the overlaps, target by target
+  // the overlaps, target by target; an infinity or a NaN in a layer makes its share NaN
+  auto tan = [&](int k) -> double { return ODD && inf_or_nan(C.q[k]) ? kNaN : C.t[k]; };
   auto mean = [&](int k, double x1, double x2) {
     const double m = 0.5 * (x1 + x2);
     return C.tl[k] + m * ((C.tr[k] - C.tl[k]) + C.t6[k]) - C.t6[k] * ((x2 * x2 + x1 * x2 + x1 * x1) * (1.0 / 3.0));
@@ -1220,9 +1348,9 @@ __global__ void __launch_bounds__(64) k_remap_tl4_state(const double* q, const d
     if (inside) {
       out = Xt == 0.0 && (Lb == Lt + 1 || Xb == 1.0) ? C.t[Lt] : mean(Lt, Xt, Lb == Lt ? Xb : 1.0);
     } else {
-      double m = Xt == 0.0 ? C.t[Lt] * C.h[Lt] : (C.h[Lt] * (1.0 - Xt)) * mean(Lt, Xt, 1.0);
-      for (int k = Lt + 1; k < Lb; ++k) m = fma(C.t[k], C.h[k], m);
-      if (Xb >= 1.0) m = fma(C.t[Lb], C.h[Lb] * Xb, m);
+      double m = Xt == 0.0 ? tan(Lt) * C.h[Lt] : (C.h[Lt] * (1.0 - Xt)) * mean(Lt, Xt, 1.0);
+      for (int k = Lt + 1; k < Lb; ++k) m = fma(tan(k), C.h[k], m);
+      if (Xb >= 1.0) m = fma(tan(Lb), C.h[Lb] * Xb, m);
       else if (Xb > 0.0) m = fma(C.h[Lb] * Xb, mean(Lb, 0.0, Xb), m);
       out = fast_div(m, pn - pe);
     }
@@ -1244,7 +1372,7 @@ __global__ void __launch_bounds__(64) k_remap_ad_rows(const double* q1, const do
   auto p1 = [&](int k) { return pe1[(long long)k * ncol + col]; };
   auto p2 = [&](int k) { return pe2[(long long)k * ncol + col]; };
   auto g2 = [&](int k2) { return q2_ad[(long long)k2 * ncol + col]; };
-  column_ad4(C, km, kn, iv, 0.0, qs ? qs[col] : 0.0, p1, p2, g2);
+  column_ad4<true>(C, km, kn, iv, 0.0, qs ? qs[col] : 0.0, p1, p2, g2);
   for (int k = 0; k < km; ++k) q1_ad[(long long)k * ncol + col] += C.qa[k];
 }
 
@@ -1276,6 +1404,7 @@ int lin_unpack_tangent(const Dual<double>* in, double* d, long long n, cudaStrea
 
 int lin_trajectory(const LinArgs& a, const double* q, const LinTraj& tr, cudaStream_t s) {
   const dim3 g = plane_grid(a);
+  FV3G_CUDA(cudaMemsetAsync(a.odd, 0, sizeof(int), s));
   if (a.dr) k_lin_ratios<<<dim3(g.x, (unsigned)(a.nt * a.npz)), 128, 0, s>>>(a);
   k_lin_corners<<<g, 128, 0, s>>>(a, q, tr.qc1, tr.qc2);
   const int lines = std::max(a.ied - a.isd, a.jed - a.jsd) + 1;
@@ -1283,9 +1412,11 @@ int lin_trajectory(const LinArgs& a, const double* q, const LinTraj& tr, cudaStr
   const bool edges = a.ew != NO_EDGE || a.ee != NO_EDGE || a.es != NO_EDGE || a.en != NO_EDGE;
   k_lin_inner<<<g, 128, 0, s>>>(a, tr);
   if (edges) k_lin_edges<<<ge, 128, 0, s>>>(a, tr, 0);
+  k_lin_odd<<<152 * 4, 128, 0, s>>>(a, tr, 0);
   k_lin_mid<<<g, 128, 0, s>>>(a, tr.qc1, tr.qc2, tr.fx2, tr.fy2, tr.qi, tr.qj);
   k_lin_outer<<<g, 128, 0, s>>>(a, tr);
   if (edges) k_lin_edges<<<ge, 128, 0, s>>>(a, tr, 1);
+  k_lin_odd<<<152 * 4, 128, 0, s>>>(a, tr, 1);
   FV3G_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1351,25 +1482,29 @@ LinArgs lin_state_args(const PlaneGeom& pg, long long P, int n, int nt, int nq, 
 
 int lin_remap_ad(const double* q, const double* dp, const double* ak, const double* bk, const double* q2_ad,
                  double* q_ad, PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv,
-                 double q_min, int kord, cudaStream_t s) {
+                 double q_min, int kord, int* odd, cudaStream_t s) {
   if (kord != 4) return set_error(FV3G_E_UNSUPPORTED, "the hand-written remap adjoint is kord 4 (got %d)", kord);
   if (km < 3 || km > KMAX || kn < 1 || kn > KMAX)
     return set_error(FV3G_E_ARG, "remap adjoint supports 3..%d layers (km=%d, kn=%d)", KMAX, km, kn);
   const long long nthr = (long long)nt * n * n * nq;
-  k_remap_ad_state<<<(unsigned)((nthr + 63) / 64), 64, 0, s>>>(q, dp, ak, bk, q2_ad, q_ad, pg, P, n, nt, nq, km, kn,
-                                                               iv, iv == 1 ? q_min : 0.0);
+  FV3G_CUDA(cudaMemsetAsync(odd, 0, sizeof(int), s));
+  for (auto kern : {k_remap_ad_state<false>, k_remap_ad_state<true>})  // the second: columns that the first reported
+    kern<<<(unsigned)((nthr + 63) / 64), 64, 0, s>>>(q, dp, ak, bk, q2_ad, q_ad, pg, P, n, nt, nq, km, kn, iv,
+                                                     iv == 1 ? q_min : 0.0, odd);
   FV3G_CUDA(cudaGetLastError());
   return 0;
 }
 
 int lin_remap_tl4(const double* q, const double* dq, const double* dp, const double* ak, const double* bk, double* dq2,
-                  PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv, double q_min,
+                  PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv, double q_min, int* odd,
                   cudaStream_t s) {
   if (km < 2 || km > KMAX || kn < 1 || kn > KMAX)
     return set_error(FV3G_E_ARG, "remap supports 2..%d layers (km=%d, kn=%d)", KMAX, km, kn);
   const long long nthr = (long long)nt * n * n * nq;
-  k_remap_tl4_state<<<(unsigned)((nthr + 63) / 64), 64, 0, s>>>(q, dq, dp, ak, bk, dq2, pg, P, n, nt, nq, km, kn, iv,
-                                                                iv == 1 ? q_min : 0.0);
+  FV3G_CUDA(cudaMemsetAsync(odd, 0, sizeof(int), s));
+  for (auto kern : {k_remap_tl4_state<false>, k_remap_tl4_state<true>})
+    kern<<<(unsigned)((nthr + 63) / 64), 64, 0, s>>>(q, dq, dp, ak, bk, dq2, pg, P, n, nt, nq, km, kn, iv,
+                                                     iv == 1 ? q_min : 0.0, odd);
   FV3G_CUDA(cudaGetLastError());
   return 0;
 }

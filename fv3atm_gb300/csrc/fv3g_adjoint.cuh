@@ -43,6 +43,7 @@ struct LinArgs {
   const double *dp1, *dp2;    // layer thickness at the substep's start and end
   double *dr, *r2;            // six-tile state: work planes dp1/dp2 and rarea/dp2 (lin_trajectory forms them)
   const double *area, *rarea, *dxa, *dya;
+  int* odd;  // work word: a window of the trajectory holds an infinity or a NaN
 };
 
 // Trajectory of one substep and its face weights (all planes at once).
@@ -89,7 +90,7 @@ int lin_fluxes_ad(const LinArgs& a, const LinTraj& tr, const LinWork& w, const d
 // read only.  iv: map1_ppm's iv (-1..1); q_min: the floor of iv 1.
 int lin_remap_ad(const double* q, const double* dp, const double* ak, const double* bk, const double* q2_ad,
                  double* q_ad, PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv,
-                 double q_min, int kord, cudaStream_t s);
+                 double q_min, int kord, int* odd, cudaStream_t s);  // odd: a work word
 
 // The hand-written column adjoint of the drop-in map1_ppm (kord 4): one row
 // of columns in [level][column] layout, pe1/pe2 the interface pressures;
@@ -99,7 +100,7 @@ int lin_remap_ad_rows(const double* q1, const double* pe1, const double* pe2, co
 
 // Tangent-linear of the same remap (kord 4): dq2 = J dq at the trajectory q, interior cells.
 int lin_remap_tl4(const double* q, const double* dq, const double* dp, const double* ak, const double* bk, double* dq2,
-                  PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv, double q_min,
+                  PlaneGeom pg, long long P, int n, int nt, int nq, int km, int kn, int iv, double q_min, int* odd,
                   cudaStream_t s);
 
 // (value, tangent) planes from value and tangent arrays (d may be null: zero

@@ -385,6 +385,7 @@ int fv3g_fv_tp_2d_ad(const double* q, double* q_ad, const double* crx, const dou
                     &w.ai, &w.aj, &w.gx, &w.gy, &w.fx2, &w.fy2};
   for (double** b : one) *b = g_ctx.take<double>(P);
   for (double** b : {&tr.wxi, &tr.wyi, &tr.wxo, &tr.wyo}) *b = g_ctx.take<double>(6 * P);
+  int* odd = g_ctx.take<int>(1);
   FV3G_CUDA(cudaMemsetAsync(g_ctx.arena, 0, g_ctx.used, s));
   struct Item {
     double* dst;
@@ -445,6 +446,7 @@ int fv3g_fv_tp_2d_ad(const double* q, double* q_ad, const double* crx, const dou
   a.mfx = wx; a.mfy = wy;
   a.ra_x = rx; a.ra_y = ry;
   a.area = area; a.dxa = dxa; a.dya = dya;
+  a.odd = odd;
   CHECK(lin_trajectory(a, qv, tr, s));
   CHECK(lin_fluxes_ad(a, tr, w, fxa, fya, damping ? d6x : nullptr, damping ? d6y : nullptr, qa, s));
   // q_ad += J^T (fx_ad, fy_ad) over the caller's data domain; the flux adjoints are consumed
