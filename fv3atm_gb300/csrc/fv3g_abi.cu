@@ -147,7 +147,8 @@ struct fv3g_state {
   cudaStream_t stream = nullptr;
   cudaStream_t up = nullptr, down = nullptr;  // fv3g_step_host: upload and download streams
   std::vector<cudaEvent_t> pev;               // fv3g_step_host: its events
-  cudaEvent_t xev = nullptr;                  // orders copies on a caller's stream with the state's stream
+  cudaEvent_t xev = nullptr;                  // orders work on a caller's stream with the state's stream
+  std::mutex xev_use;                         // its record and the wait for it are one step for several threads
   int q_cur = 0;      // buffer holding the latest tracer field
   int dp_start = 0;   // buffer holding dp at the start of the last substep
   int dp_end = 0;     // buffer holding dp at the end of the last substep
@@ -1042,9 +1043,9 @@ int fv3g_download(fv3g_state* st, int field, double* host) {
   return st->fp64 ? download_t<double>(st, fs, host, st->stream) : download_t<float>(st, fs, host, st->stream);
 }
 
-// Work on a caller's stream s other than the state's (a copy, a step, a mass
-// sum): after the work already queued on the state's stream (which may still
-// read or write the same fields) and before the work queued there after it.
+// Work on a caller's stream s other than the state's (a copy, a step, a linearised
+// step, a remap, a mass sum): after the work already queued on the state's stream (which may
+// still read or write the same fields) and before the work queued there after it.
 // A stream under capture is left to whoever builds the graph.
 static bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
@@ -1054,18 +1055,18 @@ static bool capturing(cudaStream_t s) {
   }
   return c != cudaStreamCaptureStatusNone;
 }
-static int xfer_begin(fv3g_state* st, cudaStream_t s) {
-  if (s == st->stream || capturing(s)) return 0;
+static int after(fv3g_state* st, cudaStream_t later, cudaStream_t earlier) {
+  const std::lock_guard<std::mutex> lock(st->xev_use);
   if (!st->xev) FV3G_CUDA(cudaEventCreateWithFlags(&st->xev, cudaEventDisableTiming));
-  FV3G_CUDA(cudaEventRecord(st->xev, st->stream));
-  FV3G_CUDA(cudaStreamWaitEvent(s, st->xev, 0));
+  FV3G_CUDA(cudaEventRecord(st->xev, earlier));
+  FV3G_CUDA(cudaStreamWaitEvent(later, st->xev, 0));
   return 0;
 }
+static int xfer_begin(fv3g_state* st, cudaStream_t s) {
+  return s == st->stream || capturing(s) ? 0 : after(st, s, st->stream);
+}
 static int xfer_end(fv3g_state* st, cudaStream_t s) {
-  if (s == st->stream || capturing(s)) return 0;
-  FV3G_CUDA(cudaEventRecord(st->xev, s));
-  FV3G_CUDA(cudaStreamWaitEvent(st->stream, st->xev, 0));
-  return 0;
+  return s == st->stream || capturing(s) ? 0 : after(st, st->stream, s);
 }
 
 int fv3g_upload_device(fv3g_state* st, int field, const void* dptr, void* stream) {
@@ -1120,10 +1121,7 @@ int fv3g_tracer_2d_batched(fv3g_state* st, int q_split, void* stream) {
   return xfer_end(st, s);
 }
 
-int fv3g_state_step_tl(fv3g_state* st, int q_split, int parts, const double* dq_in, double* dq_out, void* stream) {
-  if (!st || !dq_in || !dq_out) return set_error(FV3G_E_ARG, "null argument");
-  if (parts < 1 || parts > 3) return set_error(FV3G_E_ARG, "parts must be 1 (tracer_2d), 2 (remap) or 3 (both)");
-  cudaStream_t s = stream ? (cudaStream_t)stream : st->stream;
+static int step_tl_on(fv3g_state* st, int q_split, int parts, const double* dq_in, double* dq_out, cudaStream_t s) {
   CallBufs B(st, s);
   LinStep L;
   CHECK(lin_forward(st, (parts & 1) ? q_split : -1, s, B, L));
@@ -1197,11 +1195,17 @@ int fv3g_state_step_tl(fv3g_state* st, int q_split, int parts, const double* dq_
   return 0;
 }
 
-int fv3g_state_step_ad(fv3g_state* st, int q_split, int parts, const double* q_ad_out, double* q_ad_in,
-                       void* stream) {
-  if (!st || !q_ad_out || !q_ad_in) return set_error(FV3G_E_ARG, "null argument");
+int fv3g_state_step_tl(fv3g_state* st, int q_split, int parts, const double* dq_in, double* dq_out, void* stream) {
+  if (!st || !dq_in || !dq_out) return set_error(FV3G_E_ARG, "null argument");
   if (parts < 1 || parts > 3) return set_error(FV3G_E_ARG, "parts must be 1 (tracer_2d), 2 (remap) or 3 (both)");
   cudaStream_t s = stream ? (cudaStream_t)stream : st->stream;
+  CHECK(xfer_begin(st, s));
+  CHECK(step_tl_on(st, q_split, parts, dq_in, dq_out, s));
+  return xfer_end(st, s);
+}
+
+static int step_ad_on(fv3g_state* st, int q_split, int parts, const double* q_ad_out, double* q_ad_in,
+                      cudaStream_t s) {
   CallBufs B(st, s);
   LinStep L;
   CHECK(lin_forward(st, (parts & 1) ? q_split : -1, s, B, L));
@@ -1231,6 +1235,16 @@ int fv3g_state_step_ad(fv3g_state* st, int q_split, int parts, const double* q_a
   return 0;
 }
 
+int fv3g_state_step_ad(fv3g_state* st, int q_split, int parts, const double* q_ad_out, double* q_ad_in,
+                       void* stream) {
+  if (!st || !q_ad_out || !q_ad_in) return set_error(FV3G_E_ARG, "null argument");
+  if (parts < 1 || parts > 3) return set_error(FV3G_E_ARG, "parts must be 1 (tracer_2d), 2 (remap) or 3 (both)");
+  cudaStream_t s = stream ? (cudaStream_t)stream : st->stream;
+  CHECK(xfer_begin(st, s));
+  CHECK(step_ad_on(st, q_split, parts, q_ad_out, q_ad_in, s));
+  return xfer_end(st, s);
+}
+
 int fv3g_state_remap_fields(fv3g_state* st, const void* fields_in, void* fields_out, int nfield, int kind, int iv,
                             int kord, double q_min, int log_p, void* stream) {
   if (!st || !fields_in || !fields_out) return set_error(FV3G_E_ARG, "null argument");
@@ -1242,8 +1256,10 @@ int fv3g_state_remap_fields(fv3g_state* st, const void* fields_in, void* fields_
   if (kord != 4 && kord != 9) return set_error(FV3G_E_UNSUPPORTED, "kord %d not implemented (4 and 9 are)", kord);
   if (!st->levels_set) return set_error(FV3G_E_ARG, "fv3g_state_set_levels has not been called");
   cudaStream_t s = stream ? (cudaStream_t)stream : st->stream;
-  return st->fp64 ? remap_fields_t<double>(st, fields_in, fields_out, nfield, kind, iv, kord, q_min, log_p, s)
-                  : remap_fields_t<float>(st, fields_in, fields_out, nfield, kind, iv, kord, q_min, log_p, s);
+  CHECK(xfer_begin(st, s));
+  CHECK(st->fp64 ? remap_fields_t<double>(st, fields_in, fields_out, nfield, kind, iv, kord, q_min, log_p, s)
+                 : remap_fields_t<float>(st, fields_in, fields_out, nfield, kind, iv, kord, q_min, log_p, s));
+  return xfer_end(st, s);
 }
 
 int fv3g_state_nsplt(fv3g_state* st, int* nsplt) {
@@ -1733,7 +1749,11 @@ int fv3g_step_host(fv3g_state* st, int q_split, const void* q_in, const void* de
   cudaStream_t caller = stream ? (cudaStream_t)stream : st->stream;
   cudaStream_t cs = st->stream, us = st->up, ds = st->down;
   cudaEvent_t ev_start = st->pev[0], ev_lev = st->pev[1], ev_end = st->pev[need];
-  // everything after the caller's prior work on its stream
+  // everything after the caller's prior work on its stream, and after the work queued on the state's
+  if (caller != cs) {
+    CHECK(after(st, us, cs));
+    CHECK(after(st, ds, cs));
+  }
   FV3G_CUDA(cudaEventRecord(ev_start, caller));
   FV3G_CUDA(cudaStreamWaitEvent(us, ev_start, 0));
   FV3G_CUDA(cudaStreamWaitEvent(cs, ev_start, 0));
@@ -1820,7 +1840,8 @@ int fv3g_step_host(fv3g_state* st, int q_split, const void* q_in, const void* de
       CHECK(q_group_copy(st, g0, ng, q_out, true, ds, kCopyCtas, t, t + 1));
     }
   }
-  // join the three streams into the caller's
+  // join the three streams into the caller's; later work on the state's stream waits for the downloads too
+  if (caller != cs) CHECK(after(st, cs, ds));
   FV3G_CUDA(cudaEventRecord(ev_end, ds));
   FV3G_CUDA(cudaStreamWaitEvent(caller, ev_end, 0));
   FV3G_CUDA(cudaEventRecord(ev_end, cs));

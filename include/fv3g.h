@@ -344,8 +344,8 @@ int fv3g_state_set_levels(fv3g_state* st, const double* ak, const double* bk); /
  * Every `stream` argument of this header: NULL selects the state's own
  * (non-blocking) stream; any other handle is used as given, including
  * cudaStreamLegacy ((void*)1) for the legacy default stream.  Work on a
- * stream other than the state's (copies, steps, remaps, mass sums, the
- * ensemble step) is ordered after the work already queued on the state's
+ * stream other than the state's (copies, steps, the host-array and the
+ * linearised step, remaps, mass sums, the ensemble step) is ordered after the work already queued on the state's
  * stream and before the work queued there after it; a stream under capture
  * is left to the caller that builds the graph. */
 int fv3g_upload(fv3g_state* st, int field, const double* host);
