@@ -20,7 +20,7 @@ from . import _lib
 from ._lib import DP, Bounds, Grid, NestBC, StateDesc
 
 __all__ = ["Bounds", "GridStruct", "fv_tp_2d", "tracer_2d", "tracer_2d_1L", "tracer_2d_nested", "NestBoundary",
-           "map_scalar", "map1_ppm", "map_scalar_3d", "CubeState", "bounds_for"]
+           "map_scalar", "map1_ppm", "map_scalar_3d", "CubeState", "bounds_for", "release_call_buffers"]
 
 
 def _p(a):
@@ -192,6 +192,11 @@ def pressure_vars(im, km, ptop, akap, delp, pe, peln, pk, pkz) -> None:
 def map_scalar_3d(km, pe1, q1, qs, kn, pe2, q2, i1, i2, j1, j2, ibeg, iend, jbeg, jend, nq, iv, kord, q_min) -> None:
     _lib.call("fv3g_map_scalar_3d", km, _p(pe1), _p(q1), _p(qs), kn, _p(pe2), _p(q2), i1, i2, j1, j2, ibeg, iend,
               jbeg, jend, nq, iv, kord, C.c_double(q_min))
+
+
+def release_call_buffers() -> None:
+    """Return the idle work buffers of the linearised steps and field remaps of the current device."""
+    _lib.call("fv3g_release_call_buffers")
 
 
 def _stream(stream):

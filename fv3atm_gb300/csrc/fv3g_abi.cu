@@ -13,6 +13,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -104,6 +106,68 @@ static unsigned grid_for(long long n, int block = 256) {
   return (unsigned)std::max<long long>(1, std::min<long long>(g, 152LL * 16));
 }
 
+// A device's pool of call buffers, shared by its states.  A call's buffers are taken and
+// given back in the order of its stream, so calls of several states, streams and threads
+// share it; what lies idle stays mapped up to a sixteenth of the device's memory (the rest
+// returns at the next synchronisation).  It returns when an allocation of this library
+// would fail without it (device_malloc), by fv3g_release_call_buffers, and with the last state
+// that used it.  Mapping and unmapping the buffers on every call took 6 of the 63 ms of a
+// linearised step (6 x C96, 64 levels, 4 tracers, 6 substeps: 6.6 GB) and 1.6 of the 7.7 ms
+// of the pt, u and v remaps at 6 x C192 x 127 levels.
+struct CallPool {
+  cudaMemPool_t pool = nullptr;  // stays null where the device has no pools: the calls allocate
+  explicit CallPool(int device) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    size_t idle = 0, total = 0;
+    if (cudaMemGetInfo(&idle, &total) != cudaSuccess || cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      pool = nullptr;
+      return;
+    }
+    unsigned long long keep = total / 16;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  ~CallPool() {
+    if (pool) cudaMemPoolDestroy(pool);
+  }
+  CallPool(const CallPool&) = delete;
+  CallPool& operator=(const CallPool&) = delete;
+};
+static std::mutex g_pools_use;
+static std::map<int, std::weak_ptr<CallPool>> g_pools;  // by device; the states hold them
+
+static std::shared_ptr<CallPool> call_pool(int device) {
+  const std::lock_guard<std::mutex> lock(g_pools_use);
+  std::shared_ptr<CallPool> p = g_pools[device].lock();
+  if (!p) g_pools[device] = p = std::make_shared<CallPool>(device);
+  return p;
+}
+
+bool release_call_buffers(int device) {
+  std::shared_ptr<CallPool> p;
+  {
+    const std::lock_guard<std::mutex> lock(g_pools_use);
+    const auto it = g_pools.find(device);
+    if (it != g_pools.end()) p = it->second.lock();
+  }
+  if (!p || !p->pool) return false;
+  cudaMemPoolTrimTo(p->pool, 0);
+  return true;
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  int device = 0;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess && release_call_buffers(device)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 }  // namespace fv3g
 
 using namespace fv3g;
@@ -123,7 +187,8 @@ struct fv3g_state {
   void* cx = nullptr; void* cy = nullptr; void* mfx = nullptr; void* mfy = nullptr;  // inputs (unscaled)
   void* cxs = nullptr; void* cys = nullptr; void* mfxs = nullptr; void* mfys = nullptr;  // scaled copies
   void* xfx = nullptr; void* yfx = nullptr;
-  cudaMemPool_t pool = nullptr;  // buffers of one call (CallBufs), made by the first call that needs any
+  int device = 0;                  // the device of its memory and streams
+  std::shared_ptr<CallPool> pool;  // buffers of one call (CallBufs), from the first call that needs any
   std::once_flag pool_once;
   void* lev = nullptr; void* ew = nullptr;  // FP64: the marching substep's per-level planes and edge weights (AdvArgs)
   void* dp_eul = nullptr;
@@ -196,7 +261,7 @@ int mark(fv3g_state* st, int kind, cudaStream_t s, int nkern = 1) {
 }
 
 int dalloc(fv3g_state* st, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
+  cudaError_t e = device_malloc(p, bytes);
   if (e != cudaSuccess) return cuda_error(e, "cudaMalloc");
   st->allocs.push_back(*p);
   e = cudaMemsetAsync(*p, 0, bytes, st->stream);
@@ -331,7 +396,7 @@ int ensure_stage(fv3g_state* st, size_t bytes) {
   if (st->stage) cudaFree(st->stage);
   st->stage = nullptr;
   st->stage_bytes = 0;
-  FV3G_CUDA(cudaMalloc((void**)&st->stage, bytes));
+  FV3G_CUDA(device_malloc((void**)&st->stage, bytes));
   st->stage_bytes = bytes;
   return 0;
 }
@@ -633,50 +698,32 @@ int level_field_copy(fv3g_state* st, int field, const void* host, cudaStream_t s
 }
 
 // ------------------------------------------ tangent-linear and adjoint ---
-// The state's pool of call buffers.  A call's buffers are taken and given back in the order
-// of its stream, so calls on several streams and threads share it; what lies idle stays
-// mapped up to a sixteenth of the device's memory (the rest returns at the next
-// synchronisation) and goes with the state.  Mapping and unmapping them on every call took 6
-// of the 63 ms of a linearised step (6 x C96, 64 levels, 4 tracers, 6 substeps: 6.6 GB) and
-// 1.6 of the 7.7 ms of the pt, u and v remaps at 6 x C192 x 127 levels.
-void create_pool(fv3g_state* st) {
-  cudaMemPoolProps props{};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  size_t idle = 0, total = 0;
-  if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemGetInfo(&idle, &total) != cudaSuccess ||
-      cudaMemPoolCreate(&st->pool, &props) != cudaSuccess) {
-    cudaGetLastError();
-    st->pool = nullptr;  // no pools on this device: the buffers are allocated by the call
-    return;
-  }
-  unsigned long long keep = total / 16;
-  cudaMemPoolSetAttribute(st->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-}
-
 // Device buffers of one call (linearised step, field remap), given back at its end.
 struct CallBufs {
   fv3g_state* st;
   cudaStream_t s;
   std::vector<void*> p;
+  cudaMemPool_t pool;
   CallBufs(fv3g_state* state, cudaStream_t stream) : st(state), s(stream) {
-    std::call_once(st->pool_once, create_pool, st);
+    std::call_once(st->pool_once, [state] { state->pool = call_pool(state->device); });
+    pool = st->pool->pool;
   }
   CallBufs(const CallBufs&) = delete;
   CallBufs& operator=(const CallBufs&) = delete;
   ~CallBufs() {
-    for (void* x : p) st->pool ? cudaFreeAsync(x, s) : cudaFree(x);
+    for (void* x : p) pool ? cudaFreeAsync(x, s) : cudaFree(x);
+    if (pool && !p.empty()) cudaStreamSynchronize(s);  // idle from here on for device_malloc too
   }
   template <typename T>
   int take(T** out, size_t count) {
     void* v = nullptr;
     const size_t bytes = count * sizeof(T) + 256;
-    cudaError_t e = st->pool ? cudaMallocFromPoolAsync(&v, bytes, st->pool, s) : cudaMalloc(&v, bytes);
-    if (e == cudaErrorMemoryAllocation && st->pool) {  // once more without what the pool holds in pieces
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(&v, bytes, pool, s) : cudaMalloc(&v, bytes);
+    if (e == cudaErrorMemoryAllocation && pool) {  // once more without what the pool holds in pieces
       cudaGetLastError();
       cudaStreamSynchronize(s);
-      cudaMemPoolTrimTo(st->pool, 0);
-      e = cudaMallocFromPoolAsync(&v, bytes, st->pool, s);
+      cudaMemPoolTrimTo(pool, 0);
+      e = cudaMallocFromPoolAsync(&v, bytes, pool, s);
     }
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -861,6 +908,13 @@ int fv3g_last_error(char* buf, int len) {
   return 0;
 }
 
+int fv3g_release_call_buffers(void) {
+  int device = 0;
+  FV3G_CUDA(cudaGetDevice(&device));
+  release_call_buffers(device);
+  return 0;
+}
+
 int fv3g_device_info(char* buf, int len) {
   int dev = 0;
   cudaDeviceProp p;
@@ -907,6 +961,13 @@ int fv3g_state_create(const fv3g_state_desc* desc, fv3g_state** out) {
   st->pg.jsd = 1 - NG;
   st->plane = st->pg.plane();
   build_topo(st->topo);
+  {
+    const cudaError_t de = cudaGetDevice(&st->device);
+    if (de != cudaSuccess) {
+      delete st;
+      return cuda_error(de, "cudaGetDevice");
+    }
+  }
   {
     int prc = prepare_kernels();
     if (!prc) prc = prepare_remap_kernels();
@@ -968,7 +1029,6 @@ int fv3g_state_destroy(fv3g_state* st) {
   if (st->up) cudaStreamDestroy(st->up);
   if (st->down) cudaStreamDestroy(st->down);
   for (void* p : st->allocs) cudaFree(p);
-  if (st->pool) cudaMemPoolDestroy(st->pool);
   if (st->stage) cudaFree(st->stage);
   if (st->stream) cudaStreamDestroy(st->stream);
   delete st;

@@ -99,7 +99,7 @@ int staged_copy(void* dst, size_t dpitch, size_t dslice, const void* src, size_t
       g.buf = nullptr;
       g.cap = 0;
     }
-    FV3G_CUDA(cudaMalloc(&g.buf, std::max(need, size_t(1) << 20)));
+    FV3G_CUDA(device_malloc((void**)&g.buf, std::max(need, size_t(1) << 20)));
     g.cap = std::max(need, size_t(1) << 20);
   }
   if (!g.done) FV3G_CUDA(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));

@@ -34,7 +34,7 @@ struct ThreadCtx {
       if (arena) cudaFree(arena);
       arena = nullptr;
       cap = 0;
-      FV3G_CUDA(cudaMalloc((void**)&arena, bytes));
+      FV3G_CUDA(device_malloc((void**)&arena, bytes));
       cap = bytes;
     }
     used = 0;

@@ -222,6 +222,8 @@ __device__ __forceinline__ T ppm_flux(T c, T xl, T bll, T brl, T xr, T blr, T br
   return xr + (T(1) + c) * (blr + c * (blr + brr));
 }
 
+// cudaMalloc; short of memory, once more without the idle call buffers of the device (fv3g_abi.cu)
+cudaError_t device_malloc(void** p, size_t bytes);
 int set_error(int code, const char* fmt, ...);
 int cuda_error(cudaError_t e, const char* what);
 

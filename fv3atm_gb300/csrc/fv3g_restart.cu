@@ -449,7 +449,7 @@ int ensure_staging(fv3g_ncfile* f, size_t bytes, int nsums) {
     f->stage = 0;
     for (int b = 0; b < 2; ++b) {
       FV3G_CUDA(cudaHostAlloc((void**)&f->pin[b], bytes, cudaHostAllocDefault));
-      FV3G_CUDA(cudaMalloc((void**)&f->dev[b], bytes));
+      FV3G_CUDA(device_malloc((void**)&f->dev[b], bytes));
     }
     f->stage = bytes;
   }
@@ -458,7 +458,7 @@ int ensure_staging(fv3g_ncfile* f, size_t bytes, int nsums) {
   if (f->dsum_n < nsums) {
     if (f->dsum) cudaFree(f->dsum);
     f->dsum = nullptr;
-    FV3G_CUDA(cudaMalloc((void**)&f->dsum, sizeof(unsigned long long) * nsums));
+    FV3G_CUDA(device_malloc((void**)&f->dsum, sizeof(unsigned long long) * nsums));
     f->dsum_n = nsums;
   }
   return 0;

@@ -354,6 +354,15 @@ int fv3g_download(fv3g_state* st, int field, double* host);
 int fv3g_upload_device(fv3g_state* st, int field, const void* dptr, void* stream);
 int fv3g_download_device(fv3g_state* st, int field, void* dptr, void* stream);
 
+/* fv3g_state_step_tl, fv3g_state_step_ad and fv3g_state_remap_fields take work
+ * buffers of their own (6.6 GB in a linearised step of 6 x C96, 64 levels, 4
+ * tracers and 6 substeps).  One pool per device, shared by its states, keeps
+ * up to a sixteenth of the device's memory mapped between these calls; it goes
+ * with the last state that used it, or when this library runs short of memory.
+ * This entry returns what lies idle in the current device's pool (for a host
+ * model's own allocator, say); the next call maps its buffers again. */
+int fv3g_release_call_buffers(void);
+
 /* One tracer_2d call on device data: nsplt = q_split (1..64), or with
  * q_split = 0 tracer_2d's int(1 + max |Courant|) over every tile's compute
  * cells of CX and CY (one device-to-host read, so the call waits for the
