@@ -191,6 +191,7 @@ struct fv3g_state {
   std::shared_ptr<CallPool> pool;  // buffers of one call (CallBufs), from the first call that needs any
   std::once_flag pool_once;
   void* lev = nullptr; void* ew = nullptr;  // FP64: the marching substep's per-level planes and edge weights (AdvArgs)
+  int lev_nk = 0;                           // levels of the planes (stream_level_block)
   void* dp_eul = nullptr;
   void* area = nullptr; void* rarea = nullptr; void* dxa = nullptr; void* dya = nullptr;
   void* dx = nullptr; void* dy = nullptr; void* sin4 = nullptr;
@@ -323,7 +324,9 @@ AdvArgs<T> adv_args(fv3g_state* st, int src, int dst, int dp_in, int dp_out) {
   a.dp2 = (T*)st->dp[dp_out];
   if (st->lev) {
     T** const planes[STREAM_LEVEL_PLANES] = {&a.cx1, &a.cx2, &a.cy1, &a.cy2, &a.rrx, &a.rry, &a.dpa, &a.ub};
-    for (int i = 0; i < STREAM_LEVEL_PLANES; ++i) *planes[i] = (T*)st->lev + (long long)i * st->plane * st->npz * st->nt;
+    a.lev_nk = st->lev_nk;
+    a.sLt = st->plane * st->lev_nk;
+    for (int i = 0; i < STREAM_LEVEL_PLANES; ++i) *planes[i] = (T*)st->lev + i * a.sLt * st->nt;
     a.ew = (T*)st->ew;
   }
   a.sFk = st->plane;
@@ -476,9 +479,7 @@ int substeps_t(fv3g_state* st, int nsplt, int g0, int ng, cudaStream_t s, int k0
       a.cx += lo; a.cy += lo; a.xfx += lo; a.yfx += lo; a.mfx += lo; a.mfy += lo;
       a.dp1 += lo;
       a.dp2 += lo;
-      if (st->lev)
-        for (T** p : {&a.cx1, &a.cx2, &a.cy1, &a.cy2, &a.rrx, &a.rry, &a.dpa, &a.ub}) *p += lo;
-      a.npz = nk;
+      a.npz = nk;  // (the level planes' first nk levels: each range forms its own)
     }
     a.nq = ng;
     a.warps_ring = std::min(a.warps_ring, ng);
@@ -503,10 +504,10 @@ int substeps_t(fv3g_state* st, int nsplt, int g0, int ng, cudaStream_t s, int k0
       CHECK(launch_damp<T>(a, false, s));
     }
     {
-      // FP32: the interior and the edge-ring CTAs; FP64: the level planes and the march
+      // FP32: the interior and the edge-ring CTAs; FP64: the level planes and the march, per block of levels
       const BlockMap bm = block_map(a.is, a.ie, a.js, a.je, a.npx, a.npy, a.nested);
       const int nint = bm.nbxi * bm.nbyi;
-      CHECK(mark(st, K_SUBSTEP, s, (st->fp64 ? 2 : (nint > 0) + (bm.nbx * bm.nby > nint)) + (damp ? 1 : 0)));
+      CHECK(mark(st, K_SUBSTEP, s, (st->fp64 ? 2 * ((a.npz + st->lev_nk - 1) / st->lev_nk) : (nint > 0) + (bm.nbx * bm.nby > nint)) + (damp ? 1 : 0)));
     }
     if (st->cube && st->eflux != nullptr) {
       CHECK(launch_edge_fix<T>(a, st->n, s));
@@ -803,9 +804,11 @@ int lin_forward(fv3g_state* st, int q_split, cudaStream_t s, CallBufs& B, LinSte
   a.area = (const double*)st->area; a.rarea = (const double*)st->rarea;
   a.dxa = (const double*)st->dxa; a.dya = (const double*)st->dya;
   {
-    const AdvArgs<double> f = adv_args<double>(st, 0, 0, 0, 0);  // the forward substeps' reciprocals
-    a.rrx = f.rrx;
-    a.rry = f.rry;
+    const AdvArgs<double> f = adv_args<double>(st, 0, 0, 0, 0);
+    if (f.lev_nk >= st->npz) {  // the forward substeps' reciprocals; held in blocks, they are formed again
+      a.rrx = f.rrx;
+      a.rry = f.rry;
+    }
   }
   CHECK(B.take(&a.dr, L.fn));
   CHECK(B.take(&a.r2, L.fn));
@@ -995,7 +998,6 @@ int fv3g_state_create(const fv3g_state_desc* desc, fv3g_state** out) {
   for (void** m : metrics)
     if (!rc) rc = dalloc(st, m, P * nt);
   if (!rc) rc = dalloc(st, &st->sin4, P * nt * 4);
-  if (!rc && st->fp64) rc = dalloc(st, &st->lev, fb * STREAM_LEVEL_PLANES);
   if (!rc && st->fp64) rc = dalloc(st, &st->ew, st->esz * nt * (size_t)st->pg.rows * 8);
   if (!rc && st->cube && d.edge_sync)
     rc = dalloc(st, &st->eflux, st->esz * 6 * 4 * (size_t)d.npz * d.nq * d.n);
@@ -1007,6 +1009,13 @@ int fv3g_state_create(const fv3g_state_desc* desc, fv3g_state** out) {
   if (!rc) rc = dalloc(st, (void**)&st->emax, sizeof(int) * d.nq);
   if (!rc) rc = dalloc(st, (void**)&st->cmax, sizeof(unsigned long long));
   if (!rc) rc = dalloc(st, (void**)&st->err, sizeof(int));
+  if (!rc && st->fp64) {  // last, by what is left
+    size_t idle = 0, total = 0;
+    e = cudaMemGetInfo(&idle, &total);
+    if (e != cudaSuccess) rc = cuda_error(e, "cudaMemGetInfo");
+    st->lev_nk = stream_level_block(d.npz, P * nt * STREAM_LEVEL_PLANES, idle);
+    if (!rc) rc = dalloc(st, &st->lev, P * nt * STREAM_LEVEL_PLANES * st->lev_nk);
+  }
   if (!rc) {
     e = cudaStreamSynchronize(st->stream);
     if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamSynchronize");

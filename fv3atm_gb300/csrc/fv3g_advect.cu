@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(256) k_level(const AdvArgs<double> a) {
   if (jr >= pg.rows) return;
   const int i = pg.isd + ic, j = pg.jsd + jr;
   const long long p = (long long)blockIdx.z * a.sFt + blockIdx.y * a.sFk + e, pm = (long long)blockIdx.z * a.sMt + e;
+  const long long pl = (long long)blockIdx.z * a.sLt + blockIdx.y * a.sFk + e;
   if (FIRST) {
     if (blockIdx.y == 0 && ic < 2 && !a.nested) {  // one thread per row and x edge
       const double* d = a.dxa + (long long)blockIdx.z * a.sMt + (long long)jr * pg.pitch;
@@ -285,21 +286,21 @@ __global__ void __launch_bounds__(256) k_level(const AdvArgs<double> a) {
       w[2] = 0.5 + 0.5 * wr;
       w[3] = -0.5 * wr;
     }
-    auto face = [p](double c, double* w1, double* w2) {
+    auto face = [pl](double c, double* w1, double* w2) {
       const double m = fabs(c), w = 1.0 - m, v = m * w;
-      w1[p] = w;
-      w2[p] = ((__double2hiint(w) < 0) == (c > 0.0)) ? negv(absv(v)) : absv(v);
+      w1[pl] = w;
+      w2[pl] = ((__double2hiint(w) < 0) == (c > 0.0)) ? negv(absv(v)) : absv(v);
     };
     face(a.cx[p], a.cx1, a.cx2);
     face(a.cy[p], a.cy1, a.cy2);
-    if (i >= a.is && i <= a.ie) a.rrx[p] = fast_rcp(a.area[pm] + a.xfx[p] - a.xfx[p + 1]);
-    if (j >= a.js && j <= a.je) a.rry[p] = fast_rcp(a.area[pm] + a.yfx[p] - a.yfx[p + pg.pitch]);
+    if (i >= a.is && i <= a.ie) a.rrx[pl] = fast_rcp(a.area[pm] + a.xfx[p] - a.xfx[p + 1]);
+    if (j >= a.js && j <= a.je) a.rry[pl] = fast_rcp(a.area[pm] + a.yfx[p] - a.yfx[p + pg.pitch]);
   }
   if (i < a.is || i > a.ie || j < a.js || j > a.je) return;
   const double d1 = a.dp1[p], ra = a.rarea[pm];
   const double d2 = d1 + (a.mfx[p] - a.mfx[p + 1] + a.mfy[p] - a.mfy[p + pg.pitch]) * ra;
-  a.dpa[p] = 2.0 * fast_div(d1, ra);
-  a.ub[p] = 0.5 * fast_div(ra, d2);
+  a.dpa[pl] = 2.0 * fast_div(d1, ra);
+  a.ub[pl] = 0.5 * fast_div(ra, d2);
   if (a.dp2 != nullptr) a.dp2[p] = d2;
   if (!(d2 > 0.0)) raise_error(a.err, FV3G_E_DELP);
 }
@@ -329,10 +330,24 @@ int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cud
         return set_error(FV3G_E_ARG,
                          "this precision supports 1..%d advection warps per CTA and 1..%d per edge-ring CTA (got %d, %d)",
                          mw, mw, warps, a.warps_ring);
-      const int rc = launch_level(a, first, s);
-      if (rc) return rc;
-      return hord == 8 ? launch_stream_h<8>(a, warps, s)
-                       : hord == 5 ? launch_stream_h<5>(a, warps, s) : launch_stream_h<1>(a, warps, s);
+      const int nk = a.lev_nk > 0 ? std::min(a.lev_nk, a.npz) : a.npz;
+      for (int k0 = 0; k0 < a.npz; k0 += nk) {
+        AdvArgs<double> b = a;
+        const long long lo = k0 * a.sFk;
+        b.q_in += k0 * a.sQk;
+        b.q_out += k0 * a.sQk;
+        for (const double** f : {&b.cx, &b.cy, &b.xfx, &b.yfx, &b.mfx, &b.mfy, &b.dp1}) *f += lo;
+        if (b.dp2) b.dp2 += lo;
+        b.npz_e = a.npz_e ? a.npz_e : a.npz;
+        if (b.eflux) b.eflux += (long long)k0 * a.nq * (a.npx - 1);
+        b.npz = std::min(nk, a.npz - k0);
+        const int rc = launch_level(b, first || nk < a.npz, s);
+        if (rc) return rc;
+        const int rs = hord == 8 ? launch_stream_h<8>(b, warps, s)
+                                 : hord == 5 ? launch_stream_h<5>(b, warps, s) : launch_stream_h<1>(b, warps, s);
+        if (rs) return rs;
+      }
+      return 0;
     }
   }
   switch (hord) {

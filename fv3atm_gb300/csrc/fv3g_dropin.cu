@@ -243,8 +243,15 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
   const PlaneGeom pg = plane_for(bd);
   const size_t P = (size_t)pg.plane();
   const size_t nqp = (size_t)nq * npz;
-  CHECK(g_ctx.begin(padded(P * nqp, 8) * 2 + padded(P * npz, 8) * 17 + padded(P, 8) * 14 + padded((size_t)pg.rows * 8, 8) + 256 +
-                    (nest ? 2 * padded(nl.cells * nqp, 8) + 8 * 256 : 0)));
+  const size_t need = padded(P * nqp, 8) * 2 + padded(P * npz, 8) * 9 + padded(P, 8) * 14 +
+                      padded((size_t)pg.rows * 8, 8) + 256 + (nest ? 2 * padded(nl.cells * nqp, 8) + 8 * 256 : 0);
+  // levels of the marching substep's planes: one at a time, or all if they fit (stream_level_block)
+  const size_t lev_bytes = padded(P, 8) * STREAM_LEVEL_PLANES;
+  const int lev_nk = per_level ? 1
+                     : g_ctx.cap >= need + lev_bytes * npz + 64 * 256
+                         ? npz
+                         : stream_level_block(npz, lev_bytes, g_ctx.spare(need));
+  CHECK(g_ctx.begin(need + lev_bytes * lev_nk));
   cudaStream_t s = g_ctx.stream;
   double* qa = g_ctx.take<double>(P * nqp);
   double* qb = g_ctx.take<double>(P * nqp);
@@ -253,10 +260,11 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
   double *dmx = g_ctx.take<double>(P * npz), *dmy = g_ctx.take<double>(P * npz);
   double *dxf = g_ctx.take<double>(P * npz), *dyf = g_ctx.take<double>(P * npz);
   double* lev[STREAM_LEVEL_PLANES];  // the marching substep's per-level planes
-  for (double*& l : lev) l = g_ctx.take<double>(P * npz);
-  auto level_planes = [&](AdvArgs<double>& a, long long ko) {
+  for (double*& l : lev) l = g_ctx.take<double>(P * lev_nk);
+  auto level_planes = [&](AdvArgs<double>& a) {
     double** const planes[STREAM_LEVEL_PLANES] = {&a.cx1, &a.cx2, &a.cy1, &a.cy2, &a.rrx, &a.rry, &a.dpa, &a.ub};
-    for (int i = 0; i < STREAM_LEVEL_PLANES; ++i) *planes[i] = lev[i] + ko;
+    for (int i = 0; i < STREAM_LEVEL_PLANES; ++i) *planes[i] = lev[i];
+    a.lev_nk = lev_nk;
   };
   double* ew = g_ctx.take<double>((size_t)pg.rows * 8);
   double *ddx = g_ctx.take<double>(P), *ddy = g_ctx.take<double>(P), *ddxa = g_ctx.take<double>(P);
@@ -345,7 +353,7 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
         a.sQk = PL; a.sQq = PL * npz; a.sQt = 0;
         a.cx = dcx + ko; a.cy = dcy + ko; a.xfx = dxf + ko; a.yfx = dyf + ko; a.mfx = dmx + ko; a.mfy = dmy + ko;
         a.dp1 = dpb[dpi] + ko; a.dp2 = dpb[dpo] + ko;
-        level_planes(a, ko);
+        level_planes(a);
         a.ew = ew;
         a.sFk = PL; a.sFt = 0;
         a.area = dar; a.rarea = drar; a.dxa = ddxa; a.dya = ddya; a.sMt = 0;
@@ -438,7 +446,7 @@ static int tracer_2d_impl(double* q, double* dp1, double* mfx, double* mfy, doub
     a.sQk = (long long)P; a.sQq = (long long)P * npz; a.sQt = 0;
     a.cx = dcx; a.cy = dcy; a.xfx = dxf; a.yfx = dyf; a.mfx = dmx; a.mfy = dmy;
     a.dp1 = dpb[dpi]; a.dp2 = dpb[dpo];
-    level_planes(a, 0);
+    level_planes(a);
     a.ew = ew;
     a.sFk = (long long)P; a.sFt = 0;
     a.area = dar; a.rarea = drar; a.dxa = ddxa; a.dya = ddya; a.sMt = 0;

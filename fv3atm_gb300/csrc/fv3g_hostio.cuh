@@ -27,6 +27,12 @@ struct ThreadCtx {
     if (arena) cudaFree(arena);
     if (stream) cudaStreamDestroy(stream);
   }
+  // Memory that an arena could have besides bytes.
+  size_t spare(size_t bytes) const {
+    size_t idle = 0, total = 0;
+    if (cudaMemGetInfo(&idle, &total) != cudaSuccess) return 0;
+    return idle + cap > bytes ? idle + cap - bytes : 0;
+  }
   int begin(size_t bytes) {
     if (!stream) FV3G_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     bytes += 64 * 256;

@@ -105,6 +105,9 @@ struct AdvArgs {
   // Courant numbers and area fluxes: w1 = 1 - |c| and w2 = |c| w1 of the x and y faces (w2 with the sign of w1 where
   // c > 0, else the other sign), 1/ra_x, 1/ra_y; every substep: 2 dp1/rarea and rarea/(2 dp2)
   T *cx1, *cx2, *cy1, *cy2, *rrx, *rry, *dpa, *ub;
+  long long sLt;    // their tile stride (the level stride is sFk)
+  int lev_nk;       // levels they hold (0: npz); fewer than npz: the substep goes block by block (launch_substep)
+  int npz_e;        // levels of the layout of eflux (0: npz)
   // [tile][plane row][west, east][4]: the one-sided edge value at the tile's x edges as a linear form of the cells
   // e-2..e+1 of the row (e the cell beyond the edge face; weights from dxa); once per step
   T* ew;
@@ -264,6 +267,14 @@ void prepare_substep_hord(cudaError_t& err);
 
 // Marching FP64 substep kernels, one translation unit per hord (fv3g_stream_h*.cu)
 constexpr int STREAM_LEVEL_PLANES = 8;  // per-level planes of AdvArgs (cx1 .. ub)
+// Levels of them to allocate for npz levels of level_bytes each (all eight, every tile) with idle bytes
+// of memory left: all, unless they would take more than a quarter of it.  Blocks cost the planes that a
+// step's substeps share once more per substep, and smaller launches; a state or call that fits without
+// the planes runs all the same.
+inline int stream_level_block(int npz, size_t level_bytes, size_t idle) {
+  const size_t fit = idle / 4 / level_bytes;
+  return fit >= (size_t)npz ? npz : fit < 1 ? 1 : (int)fit;
+}
 template <int HORD>
 int launch_stream_h(const AdvArgs<double>& a, int warps, cudaStream_t s);
 template <int HORD>

@@ -488,8 +488,8 @@ struct March {
     const PlaneGeom& pg = a.pg;
     const int j = j0 - 3 + m, t = blockIdx.z, k = blockIdx.y;
     // edge-flux index (((t*4 + e)*npz + k)*nq + iq)*n + s = efo + e*efe + iq*n + s
-    const long long efe = (long long)a.npz * a.nq * (a.npx - 1);
-    const long long efo = (((long long)t * 4) * a.npz + k) * a.nq * (a.npx - 1);
+    const long long efe = (long long)a.npz_e * a.nq * (a.npx - 1);
+    const long long efo = (((long long)t * 4) * a.npz_e + k) * a.nq * (a.npx - 1);
     auto lev = [&](int arr, int back) -> V {  // array arr at row m - back
       V v;
       const int rr = r - back + 4;  // 0..5: rows of the pairs p2, p1, p0
@@ -632,23 +632,23 @@ __device__ __forceinline__ void stream_body(const AdvArgs<double>& a, const Stre
     }
   }
   // ---- level rows
-  const long long fo = t * a.sFt + k * a.sFk, mo = t * a.sMt;
+  const long long fo = t * a.sFt + k * a.sFk, mo = t * a.sMt, lo = t * a.sLt + k * a.sFk;
   const int wof = i0 - 3 - pg.isd;  // plane column of window column 0 (a multiple of 16 bytes)
   const int nb = (nj + 7 + SB - 1) / SB;
   if (tid < LN) {
-    const double* p = a.cx1 + fo;
-    p = tid == LX2 ? a.cx2 + fo : p;
+    const double* p = a.cx1 + lo;
+    p = tid == LX2 ? a.cx2 + lo : p;
     p = tid == LXF ? a.xfx + fo : p;
     p = tid == LAR ? a.area + mo : p;
     p = tid == LMX ? a.mfx + fo : p;
-    p = tid == LY1 ? a.cy1 + fo : p;
-    p = tid == LY2 ? a.cy2 + fo : p;
+    p = tid == LY1 ? a.cy1 + lo : p;
+    p = tid == LY2 ? a.cy2 + lo : p;
     p = tid == LYF ? a.yfx + fo : p;
     p = tid == LMY ? a.mfy + fo : p;
-    p = tid == LDP ? a.dpa + fo : p;
-    p = tid == LRA ? a.ub + fo : p;
-    p = tid == LRX ? a.rrx + fo : p;
-    p = tid == LRY ? a.rry + fo : p;
+    p = tid == LDP ? a.dpa + lo : p;
+    p = tid == LRA ? a.ub + lo : p;
+    p = tid == LRX ? a.rrx + lo : p;
+    p = tid == LRY ? a.rry + lo : p;
     S.base[tid] = p + wof;
   }
   __syncthreads();
