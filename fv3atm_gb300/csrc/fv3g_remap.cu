@@ -28,6 +28,7 @@
 #include "fv3g_ff.cuh"
 #include "fv3g_fp64.cuh"
 #include "fv3g_internal.cuh"
+#include "fv3g_ln.cuh"
 #include "fv3g_profile.cuh"
 #include "fv3g_remap.cuh"
 
@@ -960,42 +961,6 @@ int launch_remap(const RemapArgs<T>& a, int kord, cudaStream_t s) {
 // ln_tab 11; beside a face the two columns' thicknesses are summed before the running
 // sum, and halved by the exponent.  6 x C192 x 127 levels: cells in ln p 3.73 to 1.33 ms,
 // faces 0.49 to 0.30 ms.
-constexpr int LN_N = 1024;  // table entries: one per 2^-10 of the significand
-
-// ln p by table (Tang 1990): the significand m in [0.75, 1.5) times the tabulated
-// reciprocal r of its bin leaves 1 + e with |e| < 2^-10, and ln p = k ln 2 - ln r + ln(1 +
-// e), the last as its Taylor polynomial of degree 6 (error 2^-63 relative).  k ln 2 is split so
-// that its leading part is exact; the two bins beside 1 have r = 1, which keeps the
-// result's relative error there.  Error below 1 ulp, 0.53 above 1 kPa.  Zero, negative, subnormal, infinite and NaN p
-// go to log.
-__device__ __forceinline__ double ln_tab(double p, const double2* tab) {
-  const int hi = __double2hiint(p);
-  if ((unsigned)(hi - 0x00100000) >= 0x7fe00000u) return log(p);
-  const int up = (hi >> 19) & 1;  // significand from 1.5 on: halved
-  const float kf = (float)((hi >> 20) - 1023 + up);
-  const unsigned kb = __float_as_uint(kf);
-  const double k = __hiloint2double(kf == 0.f ? 0 : (int)(((kb & 0x7fffffffu) >> 3) + (896u << 20) | (kb & 0x80000000u)),
-                                    (int)(kb << 29));
-  const double m = __hiloint2double((hi & 0x000fffff) | (up ? 0x3fe00000 : 0x3ff00000), __double2loint(p));
-  const double2 t = tab[(hi >> 10) & (LN_N - 1)];
-  const double e = fma(m, t.x, -1.0);
-  double c = fma(e, -1.0 / 6.0, 1.0 / 5.0);
-  c = fma(e, c, -1.0 / 4.0);
-  c = fma(e, c, 1.0 / 3.0);
-  c = fma(e, c, -0.5);
-  const double l = fma(e * e, c, e);
-  constexpr double LN2_HI = 0x1.62e42fefa38p-1, LN2_LO = 0x1.ef35793c7673p-45;  // ln 2: 42 bits and the rest
-  return fma(k, LN2_HI, t.y + fma(k, LN2_LO, l));
-}
-__device__ __forceinline__ void ln_table(double2* tab) {
-  for (int i = threadIdx.x; i < LN_N; i += blockDim.x) {
-    const float c = 1.f + (i + 0.5f) / LN_N;  // the bin's middle; halved from 1.5 on
-    const double r = i == 0 || i == LN_N - 1 ? 1.0 : (double)(1.f / (i >= LN_N / 2 ? 0.5f * c : c));
-    tab[i] = make_double2(r, -log(r));
-  }
-  __syncthreads();
-}
-
 template <typename T, bool LOGP, bool FACE>
 __global__ void __launch_bounds__(256) k_field_pressures(const T* dp, long long sFt, long long sFk, PlaneGeom pg, int nt,
                                                          int km, int ni, int nj, int kind, const double* ak,
