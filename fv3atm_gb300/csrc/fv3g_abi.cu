@@ -1338,9 +1338,9 @@ int fv3g_state_nsplt(fv3g_state* st, int* nsplt) {
 }
 
 // Time one substep (interior + edge-ring launches, halo fill and prologue)
-// for each candidate CTA width and keep the fastest; then the same for the
-// width of the edge-ring launch alone (its CTAs need more registers and
-// shared memory, so a narrower CTA can fit twice per SM).  Reads the home
+// for each candidate CTA width and keep the fastest; then, for FP32 states, the
+// same for the width of the edge-ring launch alone (its CTAs need more registers
+// and shared memory, so a narrower CTA can fit twice per SM).  Reads the home
 // tracer buffer and writes only scratch buffers; the logical state is
 // unchanged.
 int fv3g_state_autotune(fv3g_state* st, int* warps_out) {
@@ -1396,7 +1396,7 @@ int fv3g_state_autotune(fv3g_state* st, int* warps_out) {
       }
     }
   }
-  if (!rc && best > 0) {
+  if (!rc && best > 0 && !st->fp64) {  // (the FP64 march has no edge-ring launch)
     st->pairs = best_mode;
     st->d.warps_per_cta = best;
     for (int w : cand[best_mode]) {
@@ -1486,8 +1486,9 @@ int fv3g_state_widths(fv3g_state* st, int* warps, int* warps_ring) {
   if (!st) return set_error(FV3G_E_ARG, "null state");
   const int w = st->d.warps_per_cta > 0 ? st->d.warps_per_cta : (st->fp64 ? 5 : 10);
   if (warps) *warps = w;
-  // the edge-ring launch is capped (8 warps for FP32 states, 10 otherwise)
-  if (warps_ring) *warps_ring = std::min(st->warps_ring > 0 ? st->warps_ring : w, ring_max_warps((int)st->esz));
+  // the edge-ring launch of FP32 states is capped (8 warps); FP64 states have none
+  if (warps_ring)
+    *warps_ring = st->fp64 ? w : std::min(st->warps_ring > 0 ? st->warps_ring : w, ring_max_warps((int)st->esz));
   return 0;
 }
 

@@ -325,11 +325,9 @@ int launch_substep(const AdvArgs<T>& a, int hord, bool flux_mode, int warps, cud
   }
   if constexpr (std::is_same<T, double>::value) {
     if (!flux_mode && (hord == 8 || hord == 5 || hord == 1)) {
-      const int mw = substep_max_warps((int)sizeof(T));
-      if (warps < 1 || warps > mw || a.warps_ring < 0 || a.warps_ring > mw)
-        return set_error(FV3G_E_ARG,
-                         "this precision supports 1..%d advection warps per CTA and 1..%d per edge-ring CTA (got %d, %d)",
-                         mw, mw, warps, a.warps_ring);
+      if (warps < 1 || warps > STREAM_MAX_WARPS)
+        return set_error(FV3G_E_ARG, "this precision supports 1..%d advection warps per CTA (got %d)", STREAM_MAX_WARPS,
+                         warps);
       const int nk = a.lev_nk > 0 ? std::min(a.lev_nk, a.npz) : a.npz;
       for (int k0 = 0; k0 < a.npz; k0 += nk) {
         AdvArgs<double> b = a;

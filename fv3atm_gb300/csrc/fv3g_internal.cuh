@@ -42,9 +42,8 @@ struct Topo {
 // kernel is capped at 128 registers so that two 8-warp CTAs fit an SM.
 __host__ __device__ constexpr int ring_max_warps(int element_bytes) { return element_bytes == 4 ? 8 : 10; }
 
-// Widest advection CTA (warps) that a state of this element size accepts; the
-// marching FP64 substep takes the width as the most tracers of a CTA.
-__host__ __device__ constexpr int substep_max_warps(int element_bytes) { return element_bytes == 4 ? 10 : 6; }
+// Widest CTA of the marching FP64 substep (warps, one tracer each) that a state accepts.
+constexpr int STREAM_MAX_WARPS = 6;
 
 struct PlaneGeom {
   int pitch;  // elements per row

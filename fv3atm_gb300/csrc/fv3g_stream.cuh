@@ -48,7 +48,6 @@ namespace fv3g {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-constexpr int kStreamWarps = 8;  // widest CTA (warps, one tracer each)
 constexpr int SB = 4;            // rows per batch
 
 // Strips and chunks of a launch: ns strips of W columns, nch chunks of H rows,
@@ -727,7 +726,7 @@ __device__ __forceinline__ void stream_body(const AdvArgs<double>& a, const Stre
 }
 
 template <int HORD, int NC>
-__global__ void __launch_bounds__(32 * kStreamWarps, 1) k_stream(const AdvArgs<double> a, const StreamMap sm) {
+__global__ void __launch_bounds__(32 * STREAM_MAX_WARPS, 1) k_stream(const AdvArgs<double> a, const StreamMap sm) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StreamSmem<NC> S(smem_raw, sm.G);
   int b = blockIdx.x;
@@ -775,7 +774,7 @@ inline StreamMap stream_map(int ni, int nj, int nq, int warps, long long planes)
   const int by_regs = 8;  // warps of an SM
   const double c = NC == 1 ? 3.0 : 1.5;
   double least = 0.0;
-  for (int g = std::min(std::min(warps, kStreamWarps), nq); g >= 1; --g) {
+  for (int g = std::min(std::min(warps, STREAM_MAX_WARPS), nq); g >= 1; --g) {
     const int ng = (nq + g - 1) / g, G = (nq + ng - 1) / ng;
     const long long res = std::max<long long>(
         1, std::min<long long>(by_regs / G, (227 << 10) / (long long)(StreamSmem<NC>::bytes(G) + 1024)));
@@ -817,9 +816,9 @@ int launch_stream_h(const AdvArgs<double>& a, int warps, cudaStream_t s) {
 template <int HORD>
 void prepare_stream_h(cudaError_t& err) {
   const cudaError_t es[] = {cudaFuncSetAttribute(k_stream<HORD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)StreamSmem<1>::bytes(kStreamWarps)),
+                                                 (int)StreamSmem<1>::bytes(STREAM_MAX_WARPS)),
                             cudaFuncSetAttribute(k_stream<HORD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)StreamSmem<2>::bytes(kStreamWarps))};
+                                                 (int)StreamSmem<2>::bytes(STREAM_MAX_WARPS))};
   for (cudaError_t e : es)
     if (e != cudaSuccess && err == cudaSuccess) err = e;
 }

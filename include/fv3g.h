@@ -469,7 +469,8 @@ int fv3g_state_remap_form(fv3g_state* st, int* form);
  * the following steps. */
 int fv3g_state_set_mass_fix(fv3g_state* st, int on);
 /* The advection CTA widths in use: interior CTAs and the CTAs whose window
- * holds a cube-face edge (the autotuner may run those narrower). */
+ * holds a cube-face edge (the autotuner may run those narrower).  FP64 states have
+ * one kind of CTA: both are its width. */
 int fv3g_state_widths(fv3g_state* st, int* warps, int* warps_ring);
 /* fillz on the state's remapped tracers (every interior column and tracer). */
 int fv3g_fillz_batched(fv3g_state* st, void* stream);
