@@ -97,3 +97,19 @@ def test_batched_remap_is_the_general_form_at_extremes(cuda, km, kn, kord, extre
         ok = np.isfinite(want)
         assert rel_l2(got[ok], want[ok]) <= FP64_TOL
         assert np.array_equal(got[..., 1::2], plain[..., 1::2])  # the columns without
+
+
+@pytest.mark.parametrize("kord", [9, 4])
+def test_more_fields_than_a_launch_takes(cuda, kord):
+    """1024 fields are a launch; fields of the first, of the last of it and of the next one hold a NaN."""
+    rng = np.random.default_rng(kord)
+    km, nf = 5, 1030
+    pe1 = np.cumsum(np.vstack([np.full((1, NCOL), 10.0), rng.uniform(0.2, 2.0, (km, NCOL))]), axis=0)
+    pe2 = pe1[:1] + np.linspace(0.0, 1.0, km + 1)[:, None] * (pe1[-1:] - pe1[:1])
+    pe2[-1] = pe1[-1]
+    q = rng.uniform(-1.0, 1.0, (nf, km, NCOL))
+    q[[0, 31, 32, 1023, 1024, 1029], 2, 3] = np.nan
+    want, got = _general(pe1, q, pe2, 0, kord, 0.0, None), _batched(pe1, q, pe2, 0, kord, 0.0, None)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    ok = np.isfinite(want)
+    assert rel_l2(got[ok], want[ok]) <= FP64_TOL
