@@ -243,17 +243,13 @@ __global__ void __launch_bounds__(128) k_remap_scratch(const RemapArgs<T> a) {
 //     substitution a_u = y_u - cp_u a_{u+1}, affine maps composed in the scan.
 // The overlap schedule (source layer and fractional position of every target
 // interface) is a short walk in the warp's copy of pe1.
-// Shared arrays indexed by level take one pad element per 32 floats (16
-// doubles), so that lane l reading level 4l+j (the blocked ownership) hits
-// distinct banks.
-template <typename T>
-__host__ __device__ constexpr int pk(int k) { return k + (k >> (sizeof(T) == 8 ? 4 : 5)); }
+// The pressures, indexed by level, take one pad element per 16 doubles, so that lane l
+// reading level 4l+j (the blocked ownership) hits distinct banks.
+__host__ __device__ constexpr int pk(int k) { return k + (k >> 4); }
 
-// Fields per pass of the warp kernel: FP32 columns advance two fields at a
-// time, so the lane-to-lane scans of both interleave (the scans are latency
-// chains of shuffles); FP64 keeps one (its ring has three slots).
-template <typename T>
-__host__ __device__ constexpr int fields_per_pass() { return sizeof(T) == 4 ? 2 : 1; }
+// Fields per pass of the warp kernel: two at a time, so the lane-to-lane scans of both
+// interleave (the scans are latency chains of shuffles).
+constexpr int FP = 2;
 
 // Entry k of the parabola and mass arrays: one pad entry per four, so that lanes four
 // levels apart (16-byte entries) hit distinct banks.
@@ -261,15 +257,14 @@ __host__ __device__ constexpr int px(int k) { return k + (k >> 2); }
 
 // One 16-byte entry per source layer and field, and per source interface, so that a
 // target interface gathers its layer with one load per field.
-template <typename T, int NPL>
+template <int NPL>
 struct __align__(16) ColSmem {
-  static constexpr int FP = fields_per_pass<T>();
   float4 par[FP][px(32 * NPL)];  // sub-grid parabola: left, right edge, curvature; the layer's thickness
   union {
     float4 mass[px(32 * NPL) + 1];        // cumulative layer mass of the two fields, hi.xy lo.xy (float-float)
-    double pe1[pk<double>(32 * NPL) + 1];  // during the column's set-up
+    double pe1[pk(32 * NPL) + 1];  // during the column's set-up
   };
-  T dp[32 * NPL];
+  float dp[32 * NPL];
 };
 
 // Fields reach shared memory through a ring of RING slots, filled by
@@ -281,8 +276,7 @@ struct __align__(16) ColSmem {
 // lanes that hold them, 4 bytes of 32 different sectors per instruction, they kept the
 // load/store pipe half busy (2 fields of 6 x C192 x 127 levels 0.69 ms, 0.51 ms through
 // the slots).
-template <typename T>
-__host__ __device__ constexpr int ring_slots() { return sizeof(T) == 8 ? 3 : 4; }
+constexpr int RING = 4;
 
 // Columns (warps) per CTA of the warp remap; its threads copy one level of
 // all RCOL columns at a time (8 FP32 columns: one 32-byte sector; 4 measured
@@ -291,23 +285,21 @@ constexpr int RCOL = 8;
 
 // Slot pitch per column: room for the levels, and a residue (4 mod 32 floats) that
 // spreads the 8 columns of one copy instruction over distinct banks.
-template <typename T, int NPL>
+template <int NPL>
 __host__ __device__ constexpr int ring_pitch() {
   int p = 32 * NPL;
   while (p % 32 != 4) ++p;
   return p;
 }
 
-template <typename T, int NPL>
+template <int NPL>
 __host__ __device__ constexpr size_t remap_warp_smem() {
-  return RCOL * sizeof(ColSmem<T, NPL>) + (size_t)ring_slots<T>() * RCOL * ring_pitch<T, NPL>() * sizeof(T);
+  return RCOL * sizeof(ColSmem<NPL>) + (size_t)RING * RCOL * ring_pitch<NPL>() * sizeof(float);
 }
 
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* dst, const T* src) {
+__device__ __forceinline__ void cp_async_elem(float* dst, const float* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -317,10 +309,6 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 __device__ __forceinline__ float pow2_recip(float m) {
   const int e = (__float_as_int(m) >> 23) & 0xff;
   return __int_as_float((254 - e) << 23);
-}
-__device__ __forceinline__ double pow2_recip(double m) {
-  const long long e = (__double_as_longlong(m) >> 52) & 0x7ff;
-  return __longlong_as_double((2046 - e) << 52);
 }
 
 template <typename T>
@@ -427,14 +415,14 @@ __device__ __forceinline__ void put_levels(float* p, const float (&v)[NPL]) {
   }
 }
 
-template <typename T, int KORD, int NPL>  // T: float (FP64 columns: k_remap64)
-__global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> a) {
-  static_assert(Single<T>::value, "FP32 columns");
-  constexpr int RING = ring_slots<T>(), RP = ring_pitch<T, NPL>();
+template <int KORD, int NPL>  // FP32 columns (FP64: k_remap64)
+__global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<float> a) {
+  using T = float;
+  constexpr int RP = ring_pitch<NPL>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  ColSmem<T, NPL>& S = reinterpret_cast<ColSmem<T, NPL>*>(smem_raw)[warp];
-  T* const ring = reinterpret_cast<T*>(smem_raw + RCOL * sizeof(ColSmem<T, NPL>));
+  ColSmem<NPL>& S = reinterpret_cast<ColSmem<NPL>*>(smem_raw)[warp];
+  T* const ring = reinterpret_cast<T*>(smem_raw + RCOL * sizeof(ColSmem<NPL>));
   const int nc = (int)a.ncol;  // launch_remap checks that it fits in an int
   const int col0 = blockIdx.x * RCOL;
   // the last CTA's surplus warps repeat the last column and store nothing
@@ -474,7 +462,6 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
       if (k < nk) out[(long long)k * sk] = src[k];
     }
   };
-  constexpr int FP = fields_per_pass<T>();
   static_assert(RING >= 2 * FP && RING - FP >= 2, "two slots are free until the first pass refills them");
   // the column's thicknesses come through slot RING - 2 and leave through slot RING - 1
   if (a.pe1 == nullptr) {
@@ -494,7 +481,7 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
   if (a.pe1 != nullptr) {
 #pragma unroll
     for (int j = 0; j < NPL; ++j)
-      if (u0 + j <= km) S.pe1[pk<double>(u0 + j)] = a.pe1[(long long)(u0 + j) * nc + col];
+      if (u0 + j <= km) S.pe1[pk(u0 + j)] = a.pe1[(long long)(u0 + j) * nc + col];
   } else {
     const double ptop = a.ak[0];
     double dl[NPL], tot = 0.0;
@@ -513,22 +500,22 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
     }
     const double excl = __shfl_up_sync(0xffffffffu, tot, 1);
     double s = lane == 0 ? ptop : ptop + excl;
-    if (lane == 0) S.pe1[pk<double>(0)] = ptop;
+    if (lane == 0) S.pe1[pk(0)] = ptop;
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
       s += dl[j];
-      if (u0 + j < km) S.pe1[pk<double>(u0 + j + 1)] = s;
+      if (u0 + j < km) S.pe1[pk(u0 + j + 1)] = s;
     }
   }
   __syncwarp();
-  const double ps = S.pe1[pk<double>(km)];
+  const double ps = S.pe1[pk(km)];
   auto pe2_at = [&](int k) -> double {
     if (a.pe2 != nullptr) return a.pe2[(long long)k * nc + col];
     return __fma_rn(a.bk[k], ps, a.ak[k]);
   };
 #pragma unroll
   for (int j = 0; j < NPL; ++j)
-    if (u0 + j < km) S.dp[u0 + j] = T(S.pe1[pk<double>(u0 + j + 1)] - S.pe1[pk<double>(u0 + j)]);
+    if (u0 + j < km) S.dp[u0 + j] = T(S.pe1[pk(u0 + j + 1)] - S.pe1[pk(u0 + j)]);
   __syncwarp();
 
   // ----------------------------------------- overlap schedule, target dp
@@ -547,10 +534,10 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
     const long long pkey = dkey(p);
     p2v[j] = p;
     int k1 = min(k2, km - 1);
-    while (k1 > 0 && dkey(S.pe1[pk<double>(k1)]) > pkey) --k1;
-    while (k1 < km - 1 && dkey(S.pe1[pk<double>(k1 + 1)]) <= pkey) ++k1;
+    while (k1 > 0 && dkey(S.pe1[pk(k1)]) > pkey) --k1;
+    while (k1 < km - 1 && dkey(S.pe1[pk(k1 + 1)]) <= pkey) ++k1;
     Ls[j] = k1;
-    Xs[j] = T(float(p - S.pe1[pk<double>(k1)]) / (float)S.dp[k1]);
+    Xs[j] = T(float(p - S.pe1[pk(k1)]) / (float)S.dp[k1]);
   }
   p2v[NPL] = __shfl_down_sync(0xffffffffu, p2v[0], 1);  // 32 NPL > kn: lane 31's is never used
 #pragma unroll
@@ -879,10 +866,10 @@ __global__ void __launch_bounds__(32 * RCOL, 2) k_remap_warp(const RemapArgs<T> 
     if (fl + h < a.nfield) drain((fl + h) % RING, a.q_out + qo_c + (fl + h) * a.sQqo, a.sQk, kn);
 }
 
-template <typename T, int KORD, int NPL>
+template <int KORD, int NPL>
 static cudaError_t set_remap_attr() {
-  return cudaFuncSetAttribute(k_remap_warp<T, KORD, NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)remap_warp_smem<T, NPL>());
+  return cudaFuncSetAttribute(k_remap_warp<KORD, NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)remap_warp_smem<NPL>());
 }
 
 // Raise the dynamic shared-memory limit of the remap kernels once per process
@@ -891,32 +878,32 @@ int prepare_remap_kernels() {
   static std::once_flag once;
   static cudaError_t err = cudaSuccess;
   std::call_once(once, [] {
-    cudaError_t es[] = {set_remap_attr<float, 9, 2>(), set_remap_attr<float, 9, 3>(), set_remap_attr<float, 4, 2>(),
-                        set_remap_attr<float, 4, 3>(), set_remap_attr<float, 9, 4>(), set_remap_attr<float, 9, 5>(), set_remap_attr<float, 4, 4>(),
-                        set_remap_attr<float, 4, 5>(), prepare_remap64()};
+    cudaError_t es[] = {set_remap_attr<9, 2>(), set_remap_attr<9, 3>(), set_remap_attr<9, 4>(), set_remap_attr<9, 5>(),
+                        set_remap_attr<4, 2>(), set_remap_attr<4, 3>(), set_remap_attr<4, 4>(), set_remap_attr<4, 5>(),
+                        prepare_remap64()};
     for (cudaError_t e : es)
       if (e != cudaSuccess && err == cudaSuccess) err = e;
   });
   return err == cudaSuccess ? 0 : cuda_error(err, "cudaFuncSetAttribute(k_remap_warp)");
 }
 
-template <typename T, int KORD, int NPL>
-static cudaError_t launch_warp_npl(const RemapArgs<T>& a, cudaStream_t s) {
-  constexpr size_t smem = remap_warp_smem<T, NPL>();
+template <int KORD, int NPL>
+static cudaError_t launch_warp_npl(const RemapArgs<float>& a, cudaStream_t s) {
+  constexpr size_t smem = remap_warp_smem<NPL>();
   const unsigned nb = (unsigned)((a.ncol + RCOL - 1) / RCOL);
-  k_remap_warp<T, KORD, NPL><<<nb, 32 * RCOL, smem, s>>>(a);
+  k_remap_warp<KORD, NPL><<<nb, 32 * RCOL, smem, s>>>(a);
   return cudaGetLastError();
 }
 
 // Levels a lane holds: the fewest that hold the column, so that no lanes idle (6 x C96, kord 9:
 // 33 levels x 3 fields 0.43 ms with four, 0.26 ms with two; 64 x 4 0.45 and, with three, 0.35 ms).
-template <typename T, int KORD>
-static cudaError_t launch_warp_form(const RemapArgs<T>& a, cudaStream_t s) {
+template <int KORD>
+static cudaError_t launch_warp_form(const RemapArgs<float>& a, cudaStream_t s) {
   const int k = std::max(a.km, a.kn);
-  if (k < 32 * 2) return launch_warp_npl<T, KORD, 2>(a, s);
-  if (k < 32 * 3) return launch_warp_npl<T, KORD, 3>(a, s);
-  if (k < 32 * 4) return launch_warp_npl<T, KORD, 4>(a, s);
-  return launch_warp_npl<T, KORD, 5>(a, s);
+  if (k < 32 * 2) return launch_warp_npl<KORD, 2>(a, s);
+  if (k < 32 * 3) return launch_warp_npl<KORD, 3>(a, s);
+  if (k < 32 * 4) return launch_warp_npl<KORD, 4>(a, s);
+  return launch_warp_npl<KORD, 5>(a, s);
 }
 
 template <typename T>
@@ -942,7 +929,7 @@ int launch_remap(const RemapArgs<T>& a, int kord, cudaStream_t s) {
   } else if constexpr (std::is_same<T, double>::value) {
     FV3G_CUDA(launch_remap64(a, kord, s));
   } else {
-    const cudaError_t e = kord == 9 ? launch_warp_form<T, 9>(a, s) : launch_warp_form<T, 4>(a, s);
+    const cudaError_t e = kord == 9 ? launch_warp_form<9>(a, s) : launch_warp_form<4>(a, s);
     FV3G_CUDA(e);
   }
   FV3G_CUDA(cudaGetLastError());

@@ -706,10 +706,10 @@ __device__ __forceinline__ void stream_body(const AdvArgs<double>& a, const Stre
       const double *const ecur = S.ew + slot * (SB * 8), *const epre = S.ew + before * (SB * 8);
 #pragma unroll 1
       for (int h = 0; h < SB; h += 2) {
+        static_assert(SB == 4, "the rows four back are the same rows of the batch before");
         const int m = m0 + h;
-        const double *p0 = cur + h * ROW, *p1 = h >= 2 ? p0 - 2 * ROW : pre + (SB - 2) * ROW,
-                *p2 = h >= 4 ? p0 - 4 * ROW : pre + (SB - 4 + h) * ROW;
-        const double *e0 = ecur + h * 8, *e2 = h >= 4 ? e0 - 4 * 8 : epre + (SB - 4 + h) * 8;
+        const double *p0 = cur + h * ROW, *p1 = h ? p0 - 2 * ROW : pre + 2 * ROW, *p2 = pre + h * ROW;
+        const double *e0 = ecur + h * 8, *e2 = epre + h * 8;
         double* const pt = hist + (h & 2) * (2 * C);
         if (spec) {
           M.template row<true, 0>(m, p0, p1, p2, e0, e2, pt);
