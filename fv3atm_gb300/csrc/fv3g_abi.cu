@@ -507,7 +507,8 @@ int substeps_t(fv3g_state* st, int nsplt, int g0, int ng, cudaStream_t s, int k0
       // FP32: the interior and the edge-ring CTAs; FP64: the level planes and the march, per block of levels
       const BlockMap bm = block_map(a.is, a.ie, a.js, a.je, a.npx, a.npy, a.nested);
       const int nint = bm.nbxi * bm.nbyi;
-      CHECK(mark(st, K_SUBSTEP, s, (st->fp64 ? 2 * ((a.npz + st->lev_nk - 1) / st->lev_nk) : (nint > 0) + (bm.nbx * bm.nby > nint)) + (damp ? 1 : 0)));
+      const int adv = st->fp64 ? 2 * ((a.npz + st->lev_nk - 1) / st->lev_nk) : (nint > 0) + (bm.nbx * bm.nby > nint);
+      CHECK(mark(st, K_SUBSTEP, s, adv + (damp ? 1 : 0)));
     }
     if (st->cube && st->eflux != nullptr) {
       CHECK(launch_edge_fix<T>(a, st->n, s));

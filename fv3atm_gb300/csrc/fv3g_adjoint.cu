@@ -1074,7 +1074,9 @@ template <bool ODD, class CC, class QF, class HF>
 __device__ void column_forward4(CC& C, int km, int iv, double qs, const QF& qf, const HF& hf) {
   double p[3];
   for (int k = 0; k < km; ++k)
-    C.d[k] = k < 1 || k > km - 2 ? 0.0 : slope4_grad<ODD, CC::DUAL>(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], p);
+    C.d[k] = k < 1 || k > km - 2
+                 ? 0.0
+                 : slope4_grad<ODD, CC::DUAL>(C.q[k - 1], C.q[k], C.q[k + 1], C.h[k - 1], C.h[k], C.h[k + 1], p);
   for (int u = 0; u <= km; ++u) {
     const double dml = u >= 1 ? C.d[u - 1] : 0.0, dmr = u < km ? C.d[u] : 0.0;
     if (inner_interface(u, km) && !(ODD && odd_interface(u, km, qf, dml, dmr))) {

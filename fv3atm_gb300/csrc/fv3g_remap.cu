@@ -231,7 +231,9 @@ __global__ void __launch_bounds__(128) k_remap_scratch(const RemapArgs<T> a) {
 // Bound: issue and latency of the warp's chain (62 % of issue slots, 16 warps an SM).
 // Set-up and passes of 6 x C192 x 127 levels x 9 fields: 4.65 ms before sign tests were
 // joined without branches, the float-float sums of a pass's two fields packed, the layer
-// and mass arrays gathered in 16-byte entries and the results stored by rows; 3.30 ms now.
+// and mass arrays gathered in 16-byte entries and the results stored by rows; 3.4 ms now.
+// At the 128 registers that two CTAs an SM leave, four levels a lane (96 to 127 levels) spill 20
+// bytes at kord 9 and 112 at kord 4, five 152 and 288.
 // One warp per column; lane l owns interfaces / layers u = l*NPL .. l*NPL+NPL-1,
 // so the column's constants stay in registers for all fields.  The three
 // first-order recurrences of the column are evaluated as warp scans and then

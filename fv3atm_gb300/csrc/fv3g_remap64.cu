@@ -22,9 +22,10 @@
 // field.
 // A call's divisions (pressures, pivots, target thicknesses) take fast_rcp and
 // fast_div (fv3g_fp64.cuh), a third and a half of the FP64 instructions of an IEEE
-// division.  Measured: the remap of 6 x C96 L64 x 4 tracers, kord 4, 13.2 -> 2.4 ms
-// (with 4 layers a lane for any level count and IEEE divisions 5.6); a step of 6 x
-// C192 L127 x 9, kord 9, 238 -> 173 ms.
+// division.  Measured: the remap of 6 x C96 L64 x 4 tracers, kord 4, 13.2 -> 2.9 ms
+// (with 4 layers a lane for any level count and IEEE divisions 5.6); of 6 x C192 L127 x
+// 9, kord 9, 35 ms (a step 238 -> 172 with it).  Five layers a lane (128 levels and more)
+// spill 76 bytes at kord 9 at the 168 registers that three CTAs leave.
 #include <algorithm>
 #include <mutex>
 

@@ -30,12 +30,12 @@
 // upwind cell only, what depends on the level alone is formed once for its tracers
 // (k_level), and no cell but the strip's halo is swept twice; the windowed kernel
 // (fv3g_substep.cuh) sweeps 1.5 cells per output cell and direction.  FP32 states,
-// which instruction issue bounds, keep the windowed kernel: this march took 6.1 ms
-// there against 6.0 at 6 x C192 L127 x 9 tracers, and 11.2 against 11.1 at 6 x C384
-// L64 x 16.  Measured FP64: a step of 6 x C192 L127 x 9 tracers, n_split 3, hord 8,
-// 460 -> 238 ms; 6 x C96 L64 x 4, 6 substeps, hord 5, 42.8 -> 37.2 ms; the substep of
-// the latter 3.7 -> 2.4 ms with one linear form for ordinary and one-sided interfaces
-// and no FP64 comparison left.
+// which instruction issue bounds, keep the windowed kernel: an FP32 form of this march took
+// 6.1 ms at 6 x C192 L127 x 9 tracers and 11.2 at 6 x C384 L64 x 16, the windowed kernel
+// 6.0 and 11.1 then and 4.5 at the former since.  Measured FP64, with the remap: a step of
+// 6 x C192 L127 x 9 tracers, n_split 3, hord 8, 460 -> 172 ms, its substep 44 ms; of 6 x C96
+// L64 x 4, 6 substeps, hord 5, 42.8 -> 18.3 ms, its substep 2.45 ms (FP64 pipe 84 % busy).
+// Two columns a lane spill 40 bytes at hord 8 (255 registers).
 #pragma once
 
 #include <algorithm>

@@ -398,8 +398,8 @@ int fv3g_state_remap_fields(fv3g_state* st, const void* fields_in, void* fields_
  * Arrays are device pointers in the layout of FV3G_FIELD_Q (nt*nq*npz planes
  * of nd x nd, i fastest); only interior cells are read, and halo cells of the
  * outputs are zero.
- *   fv3g_state_step_tl: dq_out = J dq_in (kord 4 or 9: the remap runs as the
- *     remap kernel on value/tangent pairs).
+ *   fv3g_state_step_tl: dq_out = J dq_in (kord 4 or 9: the remap by closed-form
+ *     derivatives of the kord-4 column, or the remap kernel on value/tangent pairs).
  *   fv3g_state_step_ad: q_ad_in = J^T q_ad_out (hand-written reverse sweeps:
  *     the substeps' PPM stencils, copy_corners and the cube halo transposed,
  *     and the kord-4 column remap; kord 9 returns FV3G_E_UNSUPPORTED).
