@@ -34,11 +34,12 @@ __device__ __forceinline__ double scale2(double a) {
   const bool ok = 2u * (unsigned)hi - 0x00800000u < 0xff600000u;  // exponent field 4 .. 2046
   return __hiloint2double(ok ? hi + K * 0x00100000 : hi, __double2loint(a));
 }
-// |a| / 4; zero for a NaN and below 2^-1019, 2^1022 for an infinity
-__device__ __forceinline__ double quarter_mag(double a) {
-  const int hi = __double2hiint(a);
-  const bool ok = 2u * (unsigned)hi - 0x00800000u <= 0xff600000u;
-  return __hiloint2double(ok ? (hi & 0x7fffffff) - 0x00200000 : 0, ok ? __double2loint(a) : 0);
+// |a| / 4; zero below 2^-1019, an infinity as it is, a NaN as it is with keep and zero without
+__device__ __forceinline__ double quarter_mag(double a, bool keep) {
+  const int hi = __double2hiint(a), mag = hi & 0x7fffffff;
+  const unsigned t = 2u * (unsigned)hi - 0x00800000u;
+  const bool ok = t <= 0xff600000u || keep;
+  return __hiloint2double(ok ? (t < 0xff600000u ? mag - 0x00200000 : mag) : 0, ok ? __double2loint(a) : 0);
 }
 // 1 / x to within an ulp in three FP64 instructions (an IEEE division takes about
 // eleven): an FP32 reciprocal r of the significand, then r + r (e + e^2) with e = 1 -

@@ -131,17 +131,19 @@ __device__ __forceinline__ Vec<NC> veast(const Vec<NC>& a) {
 
 // Monotonized central slopes in half increments: dm, |2 dm| and the sign; dp
 // and d are the differences to the cells before and after.  Beside a NaN the slope is
-// zero, as the minimum of the numbers left has it.
+// zero, as the minimum of the numbers left has it; that of an infinite cell is |xt| / 4, or, where
+// xt is no finite number, the lesser of |d| and |dp|, infinite or NaN, as the bounds leave it.
 template <int NC>
 struct Slope {
   Vec<NC> dm, two;
-  __device__ __forceinline__ void set(const Vec<NC>& xm, const Vec<NC>& xp, const Vec<NC>& dp,
+  __device__ __forceinline__ void set(const Vec<NC>& xm, const Vec<NC>& x0, const Vec<NC>& xp, const Vec<NC>& dp,
                                       const Vec<NC>& d) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const double xt = xp[c] - xm[c];
-      const bool mono = (__double2hiint(dp[c]) ^ __double2hiint(d[c])) >= 0;
-      const double m = mag_min(quarter_mag(xt), mag_min(absv(d[c]), absv(dp[c])));
+      const bool odd = inf_or_nan(x0[c]);
+      const bool mono = (__double2hiint(dp[c]) ^ __double2hiint(d[c])) >= 0 || odd;
+      const double m = mag_min(quarter_mag(xt, odd), mag_min(absv(d[c]), absv(dp[c])));
       const double mag = mono ? m : 0.0;
       dm[c] = signed_as(mag, xt);
       two[c] = scale2<1>(mag);
@@ -294,7 +296,7 @@ struct YLine {
   bool psm[NC];
   __device__ __forceinline__ void init() {
     xa = xb = xc = dp = rl = pbr = pb0 = vzero<NC>();
-    sl.set(xa, xa, xa, xa);
+    sl.set(xa, xa, xa, xa, xa);
 #pragma unroll
     for (int c = 0; c < NC; ++c) psm[c] = true;
   }
@@ -306,7 +308,7 @@ struct YLine {
     const V d = x - xc;
     if (HORD == 8) {
       Slope<NC> s1;
-      s1.set(xb, x, dp, d);  // cell m-1
+      s1.set(xb, xc, x, dp, d);  // cell m-1
       const V u = sl.dm - s1.dm;
       V rr;
       interface_raw(dp, u, rr, rn);  // interface m-1 less cell m-2 and less cell m-1
@@ -380,7 +382,7 @@ __device__ __forceinline__ Vec<NC> x_line(const Vec<NC>& x, const FaceC<NC>& f, 
 #pragma unroll
     for (int c = 0; c < NC; ++c) de[c] = c + 1 < NC ? d[c + 1 < NC ? c + 1 : 0] : xp[NC - 1] - x[NC - 1];
     Slope<NC> s;
-    s.set(xm, xp, d, de);
+    s.set(xm, x, xp, d, de);
     const V dmw = vwest(s.dm);
     V rl, rw;  // the west interfaces less the cell and less the cell west of it
     interface_raw(d, dmw - s.dm, rw, rl);

@@ -77,6 +77,20 @@ def test_tracer_with_infinities_and_nan(cuda, prob, hord, value):
 
 
 @pytest.mark.parametrize("hord", [8, 5, 1])
+@pytest.mark.parametrize("a", ["nan", "inf", "minus_inf"])
+@pytest.mark.parametrize("b", ["nan", "inf", "minus_inf"])
+def test_tracer_with_two_of_them_near_each_other(cuda, prob, hord, a, b):
+    n = prob.n
+    for off in [(0, 1), (1, 0), (0, 2), (2, 0), (1, 1), (0, 3)]:
+        for p in [(n // 2, 28), (3, n // 2), (n // 2, 3), (n + 1, n // 2), (n // 2, n), (4, 4), (n // 2, 12)]:
+            args = _args(prob, 1)
+            q = args[0][0, 0]
+            q[p] = VALUES[a]
+            q[p[0] + off[0], p[1] + off[1]] = VALUES[b]
+            _check(prob, 1, hord, args, (off, p))
+
+
+@pytest.mark.parametrize("hord", [8, 5, 1])
 def test_courant_numbers_with_nan(cuda, prob, hord):
     for p in [(10, 11), (3, 0), (20, 20), (0, 4), (prob.n + 5, 9)]:
         args = _args(prob, 1)
