@@ -35,7 +35,7 @@
 // 6.0 and 11.1 then and 4.5 at the former since.  Measured FP64, with the remap: a step of
 // 6 x C192 L127 x 9 tracers, n_split 3, hord 8, 460 -> 172 ms, its substep 44 ms; of 6 x C96
 // L64 x 4, 6 substeps, hord 5, 42.8 -> 18.3 ms, its substep 2.45 ms (FP64 pipe 84 % busy).
-// Two columns a lane spill 40 bytes at hord 8 (255 registers).
+// Two columns a lane spill 56 bytes at hord 8 (255 registers).
 #pragma once
 
 #include <algorithm>
